@@ -2,8 +2,8 @@
 // evaluated by one CUDA graph launch (no counterpart in the reference, which
 // evaluates one UniformFmm per call).
 //
-// cdfmm_b200_batch_create runs each plan's evaluate once (which also builds
-// its tensor-core work tiles and runs the M2L autotuner), then captures every
+// cdfmm_b200_batch_create runs each plan's evaluate once (which checks its
+// arguments and builds what a first call builds), then captures every
 // plan's evaluate into one graph, each on its own stream forked from and
 // joined back to a capture stream, so the geometries are independent branches
 // that the GPU overlaps.  cdfmm_b200_batch_launch replays the graph: one
@@ -17,10 +17,10 @@
 // and the results' scale factors).  Such a group runs ONE tensor-core M2L
 // whose states are the group's problems: the graph branch of each member
 // runs gather, its near field, P2M and M2M, the group's branch packs every
-// member's multipoles as one state each and runs the M2L, writing each
-// state's locals into its own plan, and each member's branch then runs L2L
-// and L2P.  One M2L with 8-24 states keeps the tensor cores far busier than
-// 8-24 one-state M2Ls (each an 8-row group with one real state).
+// member's multipoles as one state each and runs the M2L, and each member's
+// branch then forms its locals from the group's reduced ones (its state) in
+// its L2L, and runs L2P.  One M2L with 8-24 states fills more tiles than 8-24
+// one-state M2Ls and reads the operators once.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,13 +41,10 @@ using namespace cdfmm_b200;
 // One stacked-M2L group: plans of one depth and order, one state each.
 struct StackGroup {
   std::vector<int> members;          // indices into the batch's plans
-  int Kp = 0;                        // stacked states rounded up to 8
-  void *a_hi = nullptr, *a_lo = nullptr; // packed operands [boxes + 1][Kp * Kpad] BF16
+  void *a = nullptr;                 // packed operand, state k = member k
+  float *R = nullptr;                // reduced locals of the group's M2L
   float **M_list = nullptr;          // device: member k's multipoles
-  float **L_list = nullptr;          // device: member k's locals
-  int4 *tiles = nullptr;
-  int n_tiles = 0;
-  cdfmm_b200_plan::TcShape shape{1, 2, 0};
+  M2lTcArgs m2l;                     // of the group's first plan, for the group's operand
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
   std::vector<cudaEvent_t> up;       // per member: its multipoles are complete
@@ -78,8 +75,7 @@ void destroy_batch(cdfmm_b200_batch *b) {
   for (cudaEvent_t e : b->joins)
     if (e) cudaEventDestroy(e);
   for (StackGroup &g : b->groups) {
-    for (void *q : {g.a_hi, g.a_lo, static_cast<void *>(g.M_list), static_cast<void *>(g.L_list),
-                    static_cast<void *>(g.tiles)})
+    for (void *q : {g.a, static_cast<void *>(g.R), static_cast<void *>(g.M_list)})
       if (q) cudaFree(q);
     for (cudaEvent_t e : g.up)
       if (e) cudaEventDestroy(e);
@@ -96,120 +92,40 @@ int batch_fail(int code, const std::string &msg) {
   return code;
 }
 
-// Kernel arguments of a group's stacked M2L (its first plan's operators).
-TcArgs stacked_args(const cdfmm_b200_batch *b, const StackGroup &g) {
-  const cdfmm_b200_plan *p0 = b->plans[static_cast<size_t>(g.members.front())];
-  const int node_base = level_offset(2);
-  TcArgs ta{};
-  ta.a_hi = static_cast<const uint8_t *>(g.a_hi);
-  ta.a_lo = static_cast<const uint8_t *>(g.a_lo);
-  ta.b_tiles = static_cast<const uint8_t *>(p0->tc_b);
-  set_m2l_reduction(ta, p0);
-  ta.tiles = g.tiles;
-  ta.scale_l = p0->scale_l;
-  ta.L = nullptr;
-  ta.L_list = g.L_list;
-  ta.error_flag = p0->error_flag;
-  ta.n = p0->n;
-  ta.K = static_cast<int>(g.members.size());
-  ta.Kp = g.Kp;
-  ta.Kpad = p0->tc_Kpad;
-  ta.Npad = p0->tc_Npad;
-  ta.node_base = node_base;
-  ta.zero_node = p0->n_nodes - node_base;
-  ta.stages = g.shape.stages;
-  ta.m_tiles = g.shape.m_tiles;
-  ta.fuse_n = g.shape.fuse;
-  ta.acc_stride = round_up(g.shape.fuse ? 2 * p0->tc_Npad : p0->tc_Npad, 32);
-  ta.tmem_cols = tc_tmem_columns(g.shape.m_tiles, ta.acc_stride);
-  ta.box_bytes = static_cast<uint32_t>(g.Kp) * static_cast<uint32_t>(p0->tc_Kpad) * 2u;
-  ta.wait_limit = p0->tc_wait_limit;
-  return ta;
-}
-
 void enqueue_stacked_m2l(const cdfmm_b200_batch *b, const StackGroup &g, cudaStream_t s) {
   const cdfmm_b200_plan *p0 = b->plans[static_cast<size_t>(g.members.front())];
-  const int node_base = level_offset(2);
-  launch_m2l_pack(nullptr, p0->scale_m, p0->tc_fold_off, p0->tc_fold, p0->tc_n_in, g.a_hi, g.a_lo, p0->n,
-                  static_cast<int>(g.members.size()), g.Kp,
-                  p0->tc_Kpad, p0->depth, node_base, p0->n_nodes - node_base, s, g.M_list);
-  launch_m2l_tc(stacked_args(b, g), g.n_tiles, s);
+  launch_m2l_pack(nullptr, p0->tc_fold_off, p0->tc_fold, p0->tc_n_fold, p0->tc_n_in, g.a, p0->n,
+                  static_cast<int>(g.members.size()), g.m2l.chunks, p0->depth, s, g.M_list);
+  launch_m2l_tc(g.m2l, s);
 }
 
-cudaError_t upload_tiles(StackGroup &g, int depth) {
-  const std::vector<int4> t = tc_work_tiles(depth, g.shape.m_tiles * (128 / g.Kp));
-  if (g.tiles) cudaFree(g.tiles);
-  g.tiles = nullptr;
-  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&g.tiles), t.size() * sizeof(int4));
-  // (a pageable copy may return before its DMA lands: wait for it)
-  if (e == cudaSuccess) e = cudaMemcpy(g.tiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
-  g.n_tiles = static_cast<int>(t.size());
-  return e;
-}
-
-// Sets up group g (buffers, pointer tables) and picks its pipeline shape by
-// timing every candidate of its first plan on the group's own packed
-// operands (the members' multipoles from the warm-up evaluations).
+// Sets up group g: the operand and reduced locals of its stacked M2L (its
+// first plan's operators and pipeline shape) and the members' multipole
+// pointers.
 cudaError_t prepare_group(cdfmm_b200_batch *b, StackGroup &g) {
-  cdfmm_b200_plan *p0 = b->plans[static_cast<size_t>(g.members.front())];
+  const cdfmm_b200_plan *p0 = b->plans[static_cast<size_t>(g.members.front())];
   const int K = static_cast<int>(g.members.size());
-  g.Kp = round_up(K, 8);
-  const size_t boxes = static_cast<size_t>(p0->n_nodes - level_offset(2)) + 1;
-  const size_t bytes = boxes * static_cast<size_t>(g.Kp) * p0->tc_Kpad * 2;
-  std::vector<float *> M(static_cast<size_t>(K)), L(static_cast<size_t>(K));
-  for (int k = 0; k < K; ++k) {
+  std::vector<float *> M(static_cast<size_t>(K));
+  for (int k = 0; k < K; ++k)
     M[static_cast<size_t>(k)] = b->plans[static_cast<size_t>(g.members[static_cast<size_t>(k)])]->M;
-    L[static_cast<size_t>(k)] = b->plans[static_cast<size_t>(g.members[static_cast<size_t>(k)])]->L;
-  }
-  cudaError_t e = cudaMalloc(&g.a_hi, bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&g.a_lo, bytes);
+  const int splits = cdfmm_b200_m2l_splits(p0, K);
+  cudaError_t e = cudaMalloc(&g.a, m2l_operand_bytes(p0->depth, K, p0->tc_columns[0].chunks));
+  if (e == cudaSuccess)
+    e = cudaMalloc(reinterpret_cast<void **>(&g.R), sizeof(float) * cdfmm_b200_m2l_split_floats(p0, K) * splits);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&g.M_list), K * sizeof(float *));
-  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&g.L_list), K * sizeof(float *));
   if (e == cudaSuccess) e = cudaMemcpy(g.M_list, M.data(), K * sizeof(float *), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(g.L_list, L.data(), K * sizeof(float *), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy); // the copies have landed
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy); // the copy has landed
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming);
   g.up.assign(static_cast<size_t>(K), nullptr);
   for (int k = 0; k < K && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&g.up[static_cast<size_t>(k)], cudaEventDisableTiming);
   if (e != cudaSuccess) return e;
-  // shape: the fastest candidate on this group's operands (the kernel
-  // overwrites the members' locals, which the capture rewrites anyway)
-  const int node_base = level_offset(2);
-  launch_m2l_pack(nullptr, p0->scale_m, p0->tc_fold_off, p0->tc_fold, p0->tc_n_in, g.a_hi, g.a_lo, p0->n, K, g.Kp,
-                  p0->tc_Kpad, p0->depth, node_base,
-                  p0->n_nodes - node_base, g.stream, g.M_list);
-  cudaEvent_t t0 = nullptr, t1 = nullptr;
-  e = cudaEventCreate(&t0);
-  if (e == cudaSuccess) e = cudaEventCreate(&t1);
-  float best = 0.0F;
-  int best_i = -1;
-  for (size_t c = 0; c < p0->tc_candidates.size() && e == cudaSuccess; ++c) {
-    g.shape = p0->tc_candidates[c];
-    if (g.shape.m_tiles * (128 / g.Kp) > kTcMaxTargets) continue;
-    e = upload_tiles(g, p0->depth);
-    float ms = 0.0F;
-    for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep) {
-      e = cudaEventRecord(t0, g.stream);
-      launch_m2l_tc(stacked_args(b, g), g.n_tiles, g.stream);
-      if (e == cudaSuccess) e = cudaEventRecord(t1, g.stream);
-      if (e == cudaSuccess) e = cudaEventSynchronize(t1);
-      if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, t0, t1);
-    }
-    if (e == cudaSuccess && (best_i < 0 || ms < best)) {
-      best = ms;
-      best_i = static_cast<int>(c);
-    }
+  try {
+    g.m2l = cdfmm_b200_m2l_args(p0, K, g.a, g.R, splits);
+  } catch (const std::exception &) {
+    return cudaErrorInvalidConfiguration;
   }
-  if (t0) cudaEventDestroy(t0);
-  if (t1) cudaEventDestroy(t1);
-  if (e != cudaSuccess) return e;
-  if (best_i < 0) return cudaErrorInvalidConfiguration;
-  g.shape = p0->tc_candidates[static_cast<size_t>(best_i)];
-  e = upload_tiles(g, p0->depth);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream);
-  return e;
+  return cudaSuccess;
 }
 
 // Groups plans evaluated with one state each on the tensor-core M2L by
@@ -261,8 +177,7 @@ int cdfmm_b200_batch_create(cdfmm_b200_plan *const *plans, const cdfmm_b200_eval
   b->plans.assign(plans, plans + count);
   b->args.assign(args, args + count);
   cudaError_t e = cudaSetDevice(b->device);
-  // Warm-up evaluation of every plan (tiles, autotuning, error checks; the
-  // multipoles the stacked groups time their M2L shapes on).
+  // Warm-up evaluation of every plan (error checks, first-call buffers).
   for (int i = 0; i < count && e == cudaSuccess; ++i) {
     cdfmm_b200_eval_args a = args[i];
     a.synchronize = 1;
@@ -331,7 +246,7 @@ int cdfmm_b200_batch_create(cdfmm_b200_plan *const *plans, const cdfmm_b200_eval
         cdfmm_b200_plan *p = plans[i];
         e = cudaStreamWaitEvent(p->stream, g.done, 0);
         if (e != cudaSuccess) break;
-        cdfmm_b200_stacked_downward(p, &args[i], p->stream);
+        cdfmm_b200_stacked_downward(p, &args[i], p->stream, reduced_locals(g.m2l, static_cast<int>(k)));
         e = cudaEventRecord(b->joins[static_cast<size_t>(i)], p->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->capture, b->joins[static_cast<size_t>(i)], 0);
       }

@@ -1,5 +1,4 @@
-// Far-field stages of the evaluator, FP32 SIMT: moment gather, P2M, M2M, L2L,
-// L2P (fused with the near/far combine and the unsort to user order).
+// Far-field stages of the evaluator, FP32 SIMT: moment gather, P2M, L2P (fused with the near/far combine and the unsort to user order).
 //
 // Layouts (K = states of the call):
 //   mom [ns][K]            float4 (mx, my, mz, 0), Morton-sorted, scaled by 1/scale^3
@@ -331,161 +330,6 @@ __global__ void __launch_bounds__(kP2mThreads) p2m_kernel(const float4 *__restri
       out[static_cast<long long>(a) * K + kblk + k] = ix[3] < 0 ? -v : v;
     }
     __syncthreads();
-  }
-}
-
-// ---------------------------------------------------------------------------
-// M2M for one parent level (upstream src/far_field.cpp:303-331):
-//   M_parent[alpha] = sum_children sum_{g <= alpha} A_class[g] M_child[alpha - g]
-// Stages the pair list (offsets + packed pairs) and the 8 class coefficient
-// rows of one level in shared memory.
-__device__ inline void stage_pairs(const int *pair_off, const int *pairs, const float *cf, int n, int n_pairs,
-                                   int *soff, int *spair, float *scoef) {
-  for (int q = threadIdx.x; q <= n; q += blockDim.x) soff[q] = pair_off[q];
-  for (int q = threadIdx.x; q < n_pairs; q += blockDim.x) spair[q] = pairs[q];
-  for (int q = threadIdx.x; q < 8 * n; q += blockDim.x) scoef[q] = cf[q];
-  __syncthreads();
-}
-
-// M2M, one CTA per (parent, block of Ks states): the 8 children's
-// multipoles of the block are staged in shared memory ([child][coef][state],
-// rows of Ks), then a thread forms one parent coefficient for 4
-// consecutive states: per (child, pair) one class coefficient, one pair entry
-// and one float4 of staged multipoles feed 4 FMAs.  Lanes of a warp take
-// consecutive state quads of the same coefficient (conflict-free float4
-// loads, broadcast pair/coefficient loads).
-constexpr int kShiftThreads = 256;
-
-__device__ __forceinline__ void store_quad(float *dst, const float4 &v, int valid, bool add) {
-  const float e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (j < valid) dst[j] = add ? dst[j] + e[j] : e[j];
-}
-
-__global__ void __launch_bounds__(kShiftThreads) m2m_kernel(float *__restrict__ M, const int *__restrict__ pair_off,
-                                                            const int *__restrict__ pairs,
-                                                            const float *__restrict__ coef, int n, int K,
-                                                            int parent_level, int n_pairs, int Ks) {
-  extern __shared__ float4 shp4[];
-  float *sM = reinterpret_cast<float *>(shp4);                  // [8 children][n][Ks]
-  float *scoef = sM + 8 * n * Ks;                     // [8][n]
-  int *soff = reinterpret_cast<int *>(scoef + 8 * n);
-  int *spair = soff + n + 1;
-  stage_pairs(pair_off, pairs, coef + static_cast<long long>(parent_level + 1) * 8 * n, n, n_pairs, soff, spair,
-              scoef);
-  const long long parent = blockIdx.x;
-  const int kb = blockIdx.y * Ks;
-  const int kc = min(Ks, K - kb);
-  const int nq = (kc + 3) >> 2;
-  const long long per = static_cast<long long>(n) * K;
-  const float *child0 = M + (level_offset_d(parent_level + 1) + parent * 8) * per + kb;
-  const int qpr = Ks >> 2; // float4 quads per staged row
-  if ((K & 3) == 0) {
-    // rows of 4-aligned states: one asynchronous 16-byte copy per quad (all
-    // of a thread's copies in flight at once), one division per quad
-    for (int q = threadIdx.x; q < 8 * n * qpr; q += kShiftThreads) {
-      const int cr = q / qpr; // child * n + coefficient
-      const int kq = q - cr * qpr;
-      const int c = cr / n;
-      if (4 * kq < kc)
-        cp_async16(reinterpret_cast<float4 *>(sM) + q, child0 + c * per + static_cast<long long>(cr - c * n) * K + 4 * kq);
-      else
-        reinterpret_cast<float4 *>(sM)[q] = make_float4(0, 0, 0, 0);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-  } else {
-    for (int q = threadIdx.x; q < 8 * n * Ks; q += kShiftThreads) {
-      const int cr = q / Ks;
-      const int k = q - cr * Ks;
-      sM[q] = k < kc ? child0[(cr / n) * per + static_cast<long long>(cr % n) * K + k] : 0.0F;
-    }
-  }
-  __syncthreads();
-  float *out = M + (level_offset_d(parent_level) + parent) * per + kb;
-  for (int q = threadIdx.x; q < n * nq; q += kShiftThreads) {
-    const int a = q / nq;
-    const int kq = q - a * nq;
-    const int e0 = soff[a], e1 = soff[a + 1];
-    float4 v = make_float4(0, 0, 0, 0);
-    for (int c = 0; c < 8; ++c) {
-      const float *cc = scoef + c * n;
-      const float *mc = sM + c * n * Ks + 4 * kq;
-      for (int e = e0; e < e1; ++e) {
-        const int pr = spair[e];
-        const float w = cc[pr & 0xffff];
-        const float4 m = *reinterpret_cast<const float4 *>(mc + (pr >> 16) * Ks);
-        v.x = fmaf(w, m.x, v.x);
-        v.y = fmaf(w, m.y, v.y);
-        v.z = fmaf(w, m.z, v.z);
-        v.w = fmaf(w, m.w, v.w);
-      }
-    }
-    store_quad(out + static_cast<long long>(a) * K + 4 * kq, v, kc - 4 * kq, false);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// L2L for one child level (upstream src/far_field.cpp:533-581):
-//   L_child[beta] += sum_{|beta + g| <= p} B_class[g] L_parent[beta + g]
-// One CTA per (parent, block of states): the parent's locals are staged once
-// and shifted to its 8 children; a thread adds one child coefficient for 4
-// consecutive states.
-__global__ void __launch_bounds__(kShiftThreads) l2l_kernel(float *__restrict__ L, const int *__restrict__ pair_off,
-                                                            const int *__restrict__ pairs,
-                                                            const float *__restrict__ coef, int n, int K,
-                                                            int child_level, int n_pairs, int Ks) {
-  extern __shared__ float4 shl4[];
-  float *sL = reinterpret_cast<float *>(shl4);                  // [n][Ks]
-  float *scoef = sL + n * Ks;                         // [8][n]
-  int *soff = reinterpret_cast<int *>(scoef + 8 * n);
-  int *spair = soff + n + 1;
-  stage_pairs(pair_off, pairs, coef + static_cast<long long>(child_level) * 8 * n, n, n_pairs, soff, spair, scoef);
-  const long long parent = blockIdx.x;
-  const int kb = blockIdx.y * Ks;
-  const int kc = min(Ks, K - kb);
-  const int nq = (kc + 3) >> 2;
-  const long long per = static_cast<long long>(n) * K;
-  const float *src = L + (level_offset_d(child_level - 1) + parent) * per + kb;
-  const int qpr = Ks >> 2;
-  if ((K & 3) == 0) {
-    for (int q = threadIdx.x; q < n * qpr; q += kShiftThreads) {
-      const int b = q / qpr;
-      const int kq = q - b * qpr;
-      if (4 * kq < kc)
-        cp_async16(reinterpret_cast<float4 *>(sL) + q, src + static_cast<long long>(b) * K + 4 * kq);
-      else
-        reinterpret_cast<float4 *>(sL)[q] = make_float4(0, 0, 0, 0);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-  } else {
-    for (int q = threadIdx.x; q < n * Ks; q += kShiftThreads) {
-      const int b = q / Ks;
-      const int k = q - b * Ks;
-      sL[q] = k < kc ? src[static_cast<long long>(b) * K + k] : 0.0F;
-    }
-  }
-  __syncthreads();
-  float *child0 = L + (level_offset_d(child_level) + parent * 8) * per + kb;
-  for (int q = threadIdx.x; q < 8 * n * nq; q += kShiftThreads) {
-    const int cr = q / nq; // child * n + coefficient
-    const int kq = q - cr * nq;
-    const int c = cr / n;
-    const int b = cr - c * n;
-    const float *cc = scoef + c * n;
-    float4 v = make_float4(0, 0, 0, 0);
-    for (int e = soff[b]; e < soff[b + 1]; ++e) {
-      const int pr = spair[e];
-      const float w = cc[pr & 0xffff];
-      const float4 l = *reinterpret_cast<const float4 *>(sL + (pr >> 16) * Ks + 4 * kq);
-      v.x = fmaf(w, l.x, v.x);
-      v.y = fmaf(w, l.y, v.y);
-      v.z = fmaf(w, l.z, v.z);
-      v.w = fmaf(w, l.w, v.w);
-    }
-    store_quad(child0 + c * per + static_cast<long long>(b) * K + 4 * kq, v, kc - 4 * kq, true);
   }
 }
 
@@ -1004,35 +848,6 @@ void launch_p2m(const float4 *src_rel, const float4 *mom, const int *src_off, co
                                          size_step);
 }
 
-static size_t pair_smem(int n, int n_pairs) {
-  return sizeof(int) * (static_cast<size_t>(n) + 1 + n_pairs) + sizeof(float) * 8 * static_cast<size_t>(n);
-}
-
-// State block of the shift kernels: the largest of 32, 16, 8, 4 whose staged
-// block (children for M2M) fits 48 KB of shared memory, so that several CTAs
-// per SM overlap one CTA's staging with another's arithmetic.
-static int shift_state_block(int n, int n_pairs, int K, int rows) {
-  int Ks = 32;
-  while (Ks > 4 && pair_smem(n, n_pairs) + sizeof(float) * rows * static_cast<size_t>(n) * Ks + 16 > 48 * 1024) Ks /= 2;
-  return std::min(Ks, (K + 3) & ~3);
-}
-
-void launch_m2m(float *M, const int *pair_off, const int *pairs, const float *coef, int n, int K,
-                int parent_level, int n_pairs, cudaStream_t s) {
-  const int Ks = shift_state_block(n, n_pairs, K, 8);
-  const dim3 grid(1u << (3 * parent_level), static_cast<unsigned>((K + Ks - 1) / Ks));
-  const size_t smem = pair_smem(n, n_pairs) + sizeof(float) * 8 * static_cast<size_t>(n) * Ks + 16;
-  m2m_kernel<<<grid, kShiftThreads, smem, s>>>(M, pair_off, pairs, coef, n, K, parent_level, n_pairs, Ks);
-}
-
-void launch_l2l(float *L, const int *pair_off, const int *pairs, const float *coef, int n, int K,
-                int child_level, int n_pairs, cudaStream_t s) {
-  const int Ks = shift_state_block(n, n_pairs, K, 1);
-  const dim3 grid(1u << (3 * (child_level - 1)), static_cast<unsigned>((K + Ks - 1) / Ks));
-  const size_t smem = pair_smem(n, n_pairs) + sizeof(float) * static_cast<size_t>(n) * Ks + 16;
-  l2l_kernel<<<grid, kShiftThreads, smem, s>>>(L, pair_off, pairs, coef, n, K, child_level, n_pairs, Ks);
-}
-
 size_t l2p_smem_bytes(int n, int p, int Kb) {
   const int Kbp = (Kb + 3) & ~3;
   return sizeof(float) * (static_cast<size_t>(n) * Kbp + static_cast<size_t>(n) * kL2pTargets) +
@@ -1090,9 +905,6 @@ void configure_far_kernels(size_t max_smem) {
   allow_dynamic_smem(l2p_grad_kernel, max_smem);
   allow_dynamic_smem(p2m_kernel, max_smem);
   allow_dynamic_smem(l2p_kernel, max_smem);
-  allow_dynamic_smem(m2m_kernel, max_smem);
-  allow_dynamic_smem(l2l_kernel, max_smem);
-  prefer_max_shared_carveout(l2l_kernel); // runs beside the co-resident near field
 }
 
 } // namespace cdfmm_b200

@@ -31,10 +31,20 @@ size_t p2m_smem_bytes(int n, int p, int K, int chunk);
 void launch_p2m(const float4 *src_rel, const float4 *mom, const int *src_off, const int8_t *basis,
                 float *M, int n, int p, int K, int depth, int chunk, cudaStream_t s,
                 const float4 *size = nullptr, int size_step = 0);
-void launch_m2m(float *M, const int *pair_off, const int *pairs, const float *coef, int n, int K,
-                int parent_level, int n_pairs, cudaStream_t s);
-void launch_l2l(float *L, const int *pair_off, const int *pairs, const float *coef, int n, int K,
-                int child_level, int n_pairs, cudaStream_t s);
+// M2M of one parent level and L2L of one child level (separable shifts,
+// shift_kernels.cu); coef = the plan's [(depth + 1) * 8][n] shift table.
+void launch_m2m(float *M, const float *coef, int n, int p, int K, int parent_level, cudaStream_t s);
+// red: the tensor-core M2L's reduced, unscaled locals of levels 2..depth,
+// [box][(p + 1)^2][ld states]; the L2L of every level 2..depth then
+// writes the complete locals (states k0.. of red).  Without it the shifted
+// parents are added to the locals the M2L left in L (levels 3..depth).
+struct ReducedLocals {
+  const float *R = nullptr;
+  int ld = 1, k0 = 0;
+};
+void launch_l2l(float *L, const float *coef, int n, int p, int K, int child_level, cudaStream_t s,
+                const ReducedLocals *red = nullptr);
+void configure_shift_kernels(int p, size_t max_smem);
 size_t l2p_smem_bytes(int n, int p, int Kb);
 // L2P + combine; K >= 4 writes the sorted results over `near` and then unsorts
 // them to user order (2 launches), K < 4 writes user order directly.  A state

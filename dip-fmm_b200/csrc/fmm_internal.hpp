@@ -10,6 +10,8 @@
 #include <vector>
 
 #include "cdfmm_b200.h"
+#include "far_kernels.hpp"
+#include "m2l_tc.hpp"
 
 namespace cdfmm_b200 {
 
@@ -41,11 +43,8 @@ struct HostOperators {
   int depth = 0;
   std::vector<int> ax, ay, az; // basis multi-indices in basis order
 
-  // M2M / L2L: for output coefficient a, pairs [off[a], off[a+1]) of
-  // (monomial index g, input coefficient index).  Coefficient value for
-  // (level, child class, g) is coef[(level * 8 + class) * n + g].
-  std::vector<int> m2m_off, l2l_off;
-  std::vector<int> m2m_pair_g, m2m_pair_in, l2l_pair_g, l2l_pair_in;
+  // M2M / L2L shift coefficients h^g / g! of (level, child class, g) at
+  // [(level * 8 + class) * n + g].
   std::vector<float> m2m_coef, l2l_coef; // [(depth+1) * 8][n]
 
   // Normalised M2L matrices T^(t)[beta][alpha] = D^{alpha+beta} G(t) for the
@@ -111,17 +110,19 @@ cdfmm_b200::CloseGeometry cdfmm_b200_near_geometry(const cdfmm_b200_plan *plan);
 // (their multipoles stacked as the states of one tensor-core M2L).  upward:
 // gather, the near field (forked onto the plan's near stream), P2M, M2M on s;
 // downward: L2L, the join with the near field, L2P, the status record, on s.
-namespace cdfmm_b200 {
-// Tensor-core M2L work tiles (per level, deepest first: runs of T parents, the
-// 8 parity classes of a run adjacent) and the TMEM columns of m_tiles
-// accumulators acc_stride apart.
-std::vector<int4> tc_work_tiles(int depth, int T);
-uint32_t tc_tmem_columns(int m_tiles, int acc_stride);
-} // namespace cdfmm_b200
+// Arguments of a plan's tensor-core M2L (its current shape) for K states, with
+// the packed operand at `a` and room at R for the reduced locals of
+// max_splits splits.  Throws std::runtime_error.
+cdfmm_b200::M2lTcArgs cdfmm_b200_m2l_args(const cdfmm_b200_plan *plan, int K, void *a, float *R, int max_splits);
+// Floats of one split's reduced locals for K states, and the most splits
+// the plan's own launches take for K states.
+size_t cdfmm_b200_m2l_split_floats(const cdfmm_b200_plan *plan, int K);
+int cdfmm_b200_m2l_splits(const cdfmm_b200_plan *plan, int K);
 
 extern "C" {
 void cdfmm_b200_stacked_upward(cdfmm_b200_plan *plan, const cdfmm_b200_eval_args *a, cudaStream_t s);
-void cdfmm_b200_stacked_downward(cdfmm_b200_plan *plan, const cdfmm_b200_eval_args *a, cudaStream_t s);
+void cdfmm_b200_stacked_downward(cdfmm_b200_plan *plan, const cdfmm_b200_eval_args *a, cudaStream_t s,
+                                 const cdfmm_b200::ReducedLocals &red);
 }
 
 // The opaque ABI handle.
@@ -204,8 +205,6 @@ struct cdfmm_b200_plan {
   void *ngt_b = nullptr;
 
   // operators (device)
-  int *m2m_off = nullptr, *m2m_pair = nullptr; // pair = g | (in << 16)
-  int *l2l_off = nullptr, *l2l_pair = nullptr;
   float *m2m_coef = nullptr, *l2l_coef = nullptr;
   float *m2l_T = nullptr;            // traceless FP32 sub-blocks [343][tc_n_in][m2l_ld_red] (SIMT M2L)
   int m2l_ld_red = 0;
@@ -219,26 +218,21 @@ struct cdfmm_b200_plan {
   int last_K = 0;              // states whose expansions M, L hold (from state exp_state0)
   int exp_state0 = 0;
 
-  // tensor-core M2L (split BF16): availability, shapes, buffers, tiles
+  // tensor-core M2L (split BF16): availability, operators, buffers
   bool tc_supported = false;
-  int tc_Kpad = 0, tc_Npad = 0, tc_stages = 0, tc_Kp_max = 0;
-  int tc_m_tiles = 1, tc_acc_stride = 0; // accumulators per CTA, TMEM columns apart
-  int tc_fuse = 0;                        // 1: A_hi x [B_hi | B_lo] as one N = 2 Npad MMA
-  bool tc_pinned = false;                 // shape set by cdfmm_b200_set_m2l_shape: no autotuning
-  size_t tc_tuned_budget = 0;             // shared-memory budget the current shape was chosen for
   struct TcShape {
     int m_tiles, stages, fuse;
   };
-  std::vector<TcShape> tc_candidates;     // pipeline shapes the autotuner tries
-  uint32_t tc_tmem_cols = 0;
-  void *tc_a_hi = nullptr, *tc_a_lo = nullptr; // [boxes + 1][Kp_max * Kpad] BF16
-  void *tc_b = nullptr;                        // [343][Kpad/32][2][Npad * 32] BF16 (reduced operator)
+  std::vector<TcShape> tc_candidates;     // pipeline shapes; the first is the default
+  int tc_pinned = -1;                     // shape set by cdfmm_b200_set_m2l_shape (-1: the default)
+  cdfmm_b200::M2lColumns tc_columns[2];   // operator columns, unfused and fused
+  std::shared_ptr<const cdfmm_b200::M2lOperator> tc_operator[2]; // (the fused one on first use)
+  void *tc_a = nullptr;                   // packed operand of levels 2..depth, up to 128 states
+  float *tc_R = nullptr;                  // [splits][box][(p + 1)^2][K] reduced locals
+  std::unique_ptr<cdfmm_b200::M2lTcArgs> tc_args; // of the last (K, shape); reset when the shape changes
   bool p2m_tc_ok = false;                      // tensor-core P2M configured (beside the tensor-core near field)
   int *tc_fold_off = nullptr, *tc_fold = nullptr, *tc_expand = nullptr; // traceless reduction tables
-  int tc_n_in = 0, tc_n_out = 0, tc_n_derived = 0;
-  int4 *tc_tiles = nullptr;
-  size_t tc_tiles_capacity = 0;
-  int tc_tiles_Kp = 0, tc_n_tiles = 0;
+  int tc_n_in = 0, tc_n_out = 0, tc_n_derived = 0, tc_n_fold = 0;
   int *error_flag = nullptr;                   // device: nonzero after an expired bounded wait
   bool last_m2l_tc = false;
   uint32_t tc_wait_limit = 0;                  // iterations of each M2L pipeline progress wait

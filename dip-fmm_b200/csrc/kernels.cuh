@@ -82,10 +82,15 @@ __host__ __device__ inline void demorton3(uint32_t m, int &x, int &y, int &z) {
 }
 
 #ifdef __CUDACC__
-// 16-byte asynchronous global -> shared copy (bypasses registers, so many
+// 16-byte (and 4-byte) asynchronous global -> shared copy (bypasses registers, so many
 // copies of one thread are in flight at once), its commit and wait.
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
+               "l"(gmem)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
                "l"(gmem)
                : "memory");
 }

@@ -1,44 +1,63 @@
 // M2L on the 5th-generation tensor cores (tcgen05), split BF16 with FP32
-// accumulation in tensor memory (K states per call; fewer than 8 fill an
-// 8-row group of each MMA tile with zero rows).
+// accumulation in tensor memory (any number of states K <= 128).
 //
-// For one level, parity class c and a tile of T targets (rows = target x
-// state, 128 rows = one MMA M tile), the kernel accumulates over the 189 list2
-// offsets o of class c (implicit list2, see m2l_simt.cu):
+// On one level the M2L is a convolution over the grid of parents: the 8
+// children of target parent P receive from the 8 children of its 26
+// neighbours P + s every pair that does not touch (189 of 216 per child), and
+// the matrix of a pair depends on (s, source class c', target class c) alone.
+// So one row (parent, state) and one (s, c') pair is a matrix product
 //
-//   D[(t, k), beta] += sum_alpha A_o[(t, k), alpha] * B_o[beta, alpha]
-//   A_o[(t, k), alpha] = 2^(l|alpha|) M'_alpha(t - o, state k)   (exact scaling)
-//   B_o[beta, alpha]   = T^(o)[beta][alpha] = D^{alpha+beta} G(o)
+//   D[(P, k), (c, beta)] += sum_alpha A[(P + s, k), (c', alpha)] B_{s c'}[alpha, (c, beta)]
+//   A = 2^(l|alpha|) M'_alpha (exact scaling),  B = T^(o), o = c - c' - 2 s,
 //
-// on the traceless-reduced operator (M2lTraceless): alpha runs over the
-// (p+1)^2 - 1 folded moments M' (alpha_z <= 1, the monopole left out) and
-// beta over the (p+1)^2 locals with beta_z <= 1, an exact sub-block of the
-// full matrix; each operand is split x = hi + lo in BF16 with three products
-// A_hi*B_hi + A_hi*B_lo + A_lo*B_hi (the dropped lo*lo term is ~2^-16 of the
-// product), then the epilogue forms the other locals from the trace
-// relations and stores L = 2^(l(|beta|+1)) D for all n coefficients
-// (upstream math: docs/math.md "M2L normalisation and cross-level reuse").
+// all 8 target classes side by side (touching pairs are zero columns, 10% of
+// them).  alpha runs over the (p+1)^2 - 1 folded moments M' (M2lTraceless)
+// and beta over the (p+1)^2 locals with beta_z <= 1; each operand is split
+// x = hi + lo in BF16 with three products A_hi*B_hi + A_hi*B_lo + A_lo*B_hi
+// (the dropped lo*lo term is ~2^-16 of the product).  The reduced, unscaled
+// locals go to R; the L2L pass scales them, forms the others from the trace
+// relations and adds the shifted parent (shift_kernels.cu).
+// Upstream math: docs/math.md "M2L normalisation and cross-level reuse".
 //
-// Data movement: a producer warp issues bulk async copies (cp.async.bulk, TMA
-// engine) of each source box's rows (contiguous, already in the canonical
-// no-swizzle K-major core-matrix layout written by the pack kernel) and of the
-// offset's B tile (pre-tiled on the host), completing on the stage's "full"
-// mbarrier; one thread issues tcgen05.mma from shared memory into the TMEM
-// accumulators and commits to the stage's "empty" mbarrier, which frees it.
-// A pipeline unit is one offset and one 32-wide alpha chunk, so 4-8 stages
-// fit in shared memory and copies run several units ahead of the MMAs.
+// Why this shape.  A tile of 128 rows is a box of the (x, state) x y x z grid,
+// so a neighbour's rows are the same box moved by s: one tiled TMA load with
+// zero fill at the borders brings them, for any K (one state fills the rows
+// with 128 parents; no row is padding), and the 8 target classes share them.
+// The tile of B_{s c'} (alpha chunk of 16, hi and lo) is one bulk copy.  At
+// p = 6 a chunk is 8 KB of A and 25 KB of B for 600 tensor-core cycles, about
+// what L2 delivers to an SM in that time, where one target class at a time (8
+// KB + 4 KB for 96) waited on shared memory and L2.
+// Measured, the whole M2L stage with its pack (B200; before: one target class
+// per CTA, rows padded to 8 states): depth 5, p = 6: K = 64 8.2 -> 4.9 ms, K =
+// 1 1.96 -> 0.19 ms; depth 5, p = 8, K = 64 18.5 -> 14.7 ms; depth 3, p = 5, K
+// = 3 249 -> 48 us.  At K = 64 the issued work runs at 1.3 PFLOP/s (p = 6).
+//
+// Few tiles (small trees, few states): the (s, c') pairs of a tile are split
+// over `splits` CTAs, each with its own R, summed in a fixed order by a second
+// kernel (m2l_grid chooses the count).
+//
+// Two producer warps issue the copies of each chunk into a ring of stages,
+// completing on the stage's "full" mbarrier; one lane issues tcgen05.mma
+// into the TMEM accumulator and commits to the stage's "empty" mbarrier.
 // Every wait is bounded: on expiry the kernel records an error code, stops
 // issuing, drains what it issued (those waits always keep the full limit, so
 // no copy or MMA is still in flight when the CTA exits), writes NaN into its
-// targets' locals (stale values of an earlier call never pass for results),
-// frees its TMEM and returns.
+// part of R (stale values of an earlier call never pass for results), frees
+// its TMEM and returns.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <map>
+#include <mutex>
+#include <new>
+#include <stdexcept>
+#include <string>
+#include <tuple>
 
 #include "far_kernels.hpp"
+#include "fmm_internal.hpp"
 #include "kernels.cuh"
 #include "m2l_tc.hpp"
 #include "tcgen05.cuh"
@@ -49,10 +68,12 @@ namespace {
 
 constexpr int kTcThreads = 128;
 constexpr uint32_t kWaitLimit = kTcWaitLimit; // ~2 s with the back-off below
-constexpr int kKChunk = 32;               // alphas per pipeline unit
+constexpr int kChunk = 16;                    // alphas per pipeline stage (one MMA k-step)
+constexpr uint32_t kABytes = kM2lRows * kChunk * 4u; // rows of [hi 16 | lo 16] BF16: 64 bytes each
+constexpr int kSlab = 32;                     // accumulator columns staged at a time by the epilogue
+constexpr int kSlabPitch = kSlab + 1;
 
 using tc::bulk_g2s;
-using tc::fence_proxy_async;
 using tc::instr_desc_bf16;
 using tc::mbar_expect_tx;
 using tc::mbar_init;
@@ -69,426 +90,660 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
   return tc::mbar_wait(bar, parity, limit);
 }
 
-// Pipeline unit = (offset, alpha chunk of kKChunk = 32, the last chunk
-// possibly 16 wide): up to two MMA k-steps on each of the CTA's m_tiles
-// accumulators, which share the unit's B tile.  Shared-memory operand layout
-// of a chunk of width w (no swizzle, K-major, 8x16-byte core matrices):
-//   [row group][w/8 column blocks][8 rows][8 alphas]  -> LBO 128 B, SBO w*16 B
-// for A (128 rows per M tile) and for B (Npad rows = betas).  Stage =
-// [A_hi x m_tiles][A_lo x m_tiles][B_hi][B_lo].  Global operands hold each
-// chunk in the same order, so one source box's rows of one chunk are one
-// contiguous bulk copy; lanes of the producer warp issue a unit's copies in
-// parallel.
-template <int MT>
-__global__ void __launch_bounds__(kTcThreads, 1) m2l_tc_kernel(const TcArgs args) {
+__host__ __device__ constexpr uint32_t b_tile_bytes(int cols) { return static_cast<uint32_t>(cols) * kChunk * 4u; }
+__host__ __device__ constexpr uint32_t stage_bytes_of(int cols) { return kABytes + b_tile_bytes(cols); }
+
+// MMA widths (multiples of 16, at most 256) that cover `cols` columns.
+__device__ __forceinline__ int piece_width(int cols) {
+  const int pieces = (cols + 255) / 256;
+  return ((cols / pieces + 15) / 16) * 16;
+}
+
+__global__ void __launch_bounds__(kTcThreads, 1) m2l_tc_kernel(const __grid_constant__ M2lTcArgs args) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int4 tile = args.tiles[blockIdx.x];
-  const int level = tile.x;
-  const int cls = tile.y;
-  const int p_first = tile.z; // first parent (Morton index at level-1) of this tile
-  const int count = tile.w;   // targets in this tile (<= m_tiles * 128 / Kp)
-  const int cx = cls & 1, cy = (cls >> 1) & 1, cz = (cls >> 2) & 1;
-  const int side = 1 << level;
+  const int warp = tid >> 5, lane = tid & 31;
   const int S = args.stages;
-  const int T = 128 / args.Kp;                                      // targets per M tile
-  const int m_active = (count + T - 1) / T;
-  const int nkc = (args.Kpad + kKChunk - 1) / kKChunk;
-
-  const uint32_t a_tile = 128u * kKChunk * 2u;                      // one M tile, one of hi / lo
-  const uint32_t a_bytes = a_tile * static_cast<uint32_t>(MT);
-  const uint32_t b_bytes = static_cast<uint32_t>(args.Npad) * kKChunk * 2u;
-  const uint32_t stage_bytes = 2u * a_bytes + 2u * b_bytes;
-  uint8_t *stage0 = smem;
-  // the stages, reused after the last MMA by the epilogue's full-basis rows
-  const uint32_t epi_bytes = (128u * static_cast<uint32_t>(args.n) * 4u + 15u) & ~15u;
-  const uint32_t pipe_bytes = max(static_cast<uint32_t>(S) * stage_bytes, epi_bytes);
+  const uint32_t stage_bytes = stage_bytes_of(args.cols);
+  const uint32_t pipe_bytes = max(static_cast<uint32_t>(S) * stage_bytes,
+                                  static_cast<uint32_t>(sizeof(float) * kM2lRows * kSlabPitch));
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + pipe_bytes);
-  uint64_t *empty = full + S;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(empty + S);
+  uint64_t *empty = full + kM2lMaxStages;
+  long long *seg_base = reinterpret_cast<long long *>(empty + kM2lMaxStages); // [kM2lRows] parents' rows of R (-1: none)
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(seg_base + kM2lRows);
   int *abort_flag = reinterpret_cast<int *>(tmem_slot + 1);
-  int *tgt_node = abort_flag + 1;            // [kTcMaxTargets]
-  int *tgt_xyz = tgt_node + kTcMaxTargets;   // [kTcMaxTargets] packed coordinates
-  int *act = tgt_xyz + kTcMaxTargets;        // [216] offset positions that reach a source box in the grid
-  int *n_act = act + 216;                    // their count
-  int *last_unit = n_act + 1;                // [8] per stage: the last pipeline unit issued into it
+  int *n_act = abort_flag + 1;
+  int *act = n_act + 1;                  // [kM2lShifts] neighbours with a parent in the grid
+  int *last_a = act + kM2lShifts;        // [kM2lMaxStages] the last chunk issued into each stage
+  int *last_b = last_a + kM2lMaxStages;
 
-  // Zero every stage once: A rows beyond a tile's targets are never written.
-  for (uint32_t q = tid; q < S * stage_bytes / 16u; q += kTcThreads)
-    reinterpret_cast<uint4 *>(stage0)[q] = make_uint4(0, 0, 0, 0);
-  if (tid < count) {
-    int px, py, pz;
-    demorton3(static_cast<uint32_t>(p_first + tid), px, py, pz);
-    const int tx = 2 * px + cx, ty = 2 * py + cy, tz = 2 * pz + cz;
-    tgt_node[tid] = level_offset_d(level) + static_cast<int>(morton3(tx, ty, tz));
-    tgt_xyz[tid] = tx | (ty << 10) | (tz << 20);
+  // this CTA's tile, column group and split
+  int t = blockIdx.x;
+  const int split = t % args.splits;
+  t /= args.splits;
+  const int group = t % args.groups;
+  t /= args.groups;
+  int level = args.depth;
+  for (; level > 2; --level) {
+    const M2lLevel &l = args.levels[level - 2];
+    const int count = l.tx * l.ty * l.tz;
+    if (t < count) break;
+    t -= count;
   }
-  if (tid < 8) last_unit[tid] = -1;
+  const M2lLevel lv = args.levels[level - 2];
+  const int K = args.K;
+  const int ix = t % lv.tx, iy = (t / lv.tx) % lv.ty, iz = t / (lv.tx * lv.ty);
+  const int x0 = ix * lv.bx, y0 = iy * lv.by, z0 = iz * lv.bz; // x0 in (parent x, state) units
+  const int side = lv.side;
+  const long long level_box = level_offset_d(level) - level_offset_d(2); // first box of this level
+
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], 2);
       mbar_init(&empty[s], 1);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncthreads();
-  // list2 offsets of class (cx, cy, cz): o in [c-3, c+2]^3 minus |o| <= 1, x
-  // fastest; an offset whose source box lies outside the grid for every
-  // target of the tile (zero multipoles) is dropped from the pipeline.
-  for (int i = tid; i < 216; i += kTcThreads) {
-    const int ox = cx - 3 + i % 6, oy = cy - 3 + (i / 6) % 6, oz = cz - 3 + i / 36;
-    bool use = !(ox >= -1 && ox <= 1 && oy >= -1 && oy <= 1 && oz >= -1 && oz <= 1);
-    if (use) {
-      use = false;
-      for (int t = 0; t < count && !use; ++t) {
-        const int xyz = tgt_xyz[t];
-        const int sx = (xyz & 1023) - ox, sy = ((xyz >> 10) & 1023) - oy, sz = ((xyz >> 20) & 1023) - oz;
-        use = sx >= 0 && sy >= 0 && sz >= 0 && sx < side && sy < side && sz < side;
-      }
+  if (tid < kM2lMaxStages) last_a[tid] = last_b[tid] = -1;
+  if (warp == 0) {
+    // neighbours that reach a parent inside the grid for some row
+    bool use = false;
+    if (lane < kM2lShifts && lane != kM2lShifts / 2) {
+      const int sx = lane % 3 - 1, sy = (lane / 3) % 3 - 1, sz = lane / 9 - 1;
+      const int px0 = x0 / K, px1 = min((x0 + lv.bx - 1) / K, side - 1);
+      const int py1 = min(y0 + lv.by - 1, side - 1), pz1 = min(z0 + lv.bz - 1, side - 1);
+      use = px1 + sx >= 0 && px0 + sx < side && py1 + sy >= 0 && y0 + sy < side && pz1 + sz >= 0 && z0 + sz < side;
     }
-    act[i] = use ? 1 : 0;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int c = 0;
-    for (int i = 0; i < 216; ++i)
-      if (act[i]) act[c++] = i;
-    *n_act = c;
-  }
-  fence_proxy_async();
-  if (tid < 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(args.tmem_cols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    const uint32_t m = __ballot_sync(0xffffffffu, use);
+    if (use) act[__popc(m & ((1u << lane) - 1u))] = lane;
+    if (lane == 0) *n_act = __popc(m);
+    __syncwarp();
+    tc::tmem_alloc(tmem_slot, args.tmem_cols);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const int units = *n_act * nkc;
+  // (neighbour, source class) pairs of this split, in chunks of 16 alphas
+  const int pairs = *n_act * 8;
+  const int u0 = static_cast<int>(static_cast<long long>(pairs) * split / args.splits);
+  const int u1 = static_cast<int>(static_cast<long long>(pairs) * (split + 1) / args.splits);
+  const int items = (u1 - u0) * args.chunks;
 
-  if (tid >= 32) {
-    // Producer warps 1..npw: warp 1 + w issues the bulk copies of units
-    // u = w, w + npw, ... (an (offset, chunk) pair each) into stage u % S.
-    // Several warps overlap the address arithmetic and copy issue of
-    // consecutive units.  npw <= S: a producer waiting for the previous use
-    // (u - S) of its stage knows that its own previous unit's stage wait
-    // (u - npw - S) completed, so every unit up to u - 2S has completed and
-    // the stage's empty barrier is at most one phase behind (a parity wait
-    // cannot alias an older phase).
-    const int npw = min(kTcThreads / 32 - 1, S);
-    const int pw = (tid >> 5) - 1;
-    const size_t btile = static_cast<size_t>(args.Npad) * kKChunk * 2u; // stride of one B chunk tile
-    for (int u = pw; pw < npw && u < units; u += npw) {
-      const int s = u % S;
-      int ok = 1;
-      if (lane == 0) {
-        if (u >= S && !mbar_wait(&empty[s], ((u / S) - 1) & 1, args.wait_limit)) {
-          *abort_flag = 1;
-          atomicExch(args.error_flag, 1);
+  // The three roles below run as whole warps with one lane issuing: the loop
+  // variables are then warp-uniform, and the issuing lane's per-chunk work is
+  // little more than the wait and the instruction itself.  (One thread per
+  // role, and one for both operands, spent 700 cycles of address arithmetic
+  // on each chunk, more than its MMAs take.)
+  if (warp == 1 || warp == 2) {
+    // Producers: warp 1 the rows (A), warp 2 the operator tiles (B); a stage
+    // is full when both have arrived.
+    const bool rows = warp == 1;
+    const uint32_t bytes = rows ? static_cast<uint32_t>(lv.bx * lv.by * lv.bz) * kChunk * 4u : b_tile_bytes(args.cols);
+    const CUtensorMap *map = &args.maps[level - 2];
+    int s = 0, i = 0;
+    uint32_t phase = 1; // the first pass over the ring waits for nothing
+    bool ok = true;
+    for (int u = u0; ok && u < u1; ++u) {
+      const int sh = act[u >> 3], cls = u & 7;
+      const int x = x0 + (sh % 3 - 1) * K, y = y0 + (sh / 3) % 3 - 1, z = z0 + sh / 9 - 1;
+      int alpha = cls * args.chunks * 2 * kChunk;
+      const uint8_t *tile = args.b + ((static_cast<size_t>(sh) * 8 + cls) * args.groups + group) * args.chunks *
+                                         static_cast<size_t>(b_tile_bytes(args.cols));
+      for (int chunk = 0; chunk < args.chunks; ++chunk, ++i) {
+        if (i >= S && !__all_sync(0xffffffffu, mbar_wait(&empty[s], phase, args.wait_limit))) {
+          if (lane == 0) {
+            *abort_flag = 1;
+            atomicExch(args.error_flag, 1);
+          }
+          ok = false;
+          break;
         }
-        ok = *reinterpret_cast<volatile int *>(abort_flag) == 0;
-      }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      const int kc = u % nkc;
-      const int i = act[u / nkc];
-      const int ox = cx - 3 + i % 6, oy = cy - 3 + (i / 6) % 6, oz = cz - 3 + i / 36;
-      const int slot = (ox + 3) * 49 + (oy + 3) * 7 + (oz + 3);
-      const int kcw = min(kKChunk, args.Kpad - kc * kKChunk);
-      const uint32_t box_chunk = static_cast<uint32_t>(args.Kp * kcw * 2); // one box's rows of this chunk
-      uint8_t *st = stage0 + s * stage_bytes;
-      const int n_a = count * 2;
-      if (lane == 0)
-        mbar_expect_tx(&full[s], static_cast<uint32_t>(n_a) * box_chunk + 2u * static_cast<uint32_t>(args.Npad) * kcw * 2u);
-      __syncwarp();
-      for (int c = lane; c < n_a + 2; c += 32) {
-        if (c < n_a) {
-          const int h = c & 1;
-          const int t = c >> 1;
-          const int m = t / T;
-          const int xyz = tgt_xyz[t];
-          const int sx = (xyz & 1023) - ox, sy = ((xyz >> 10) & 1023) - oy, sz = ((xyz >> 20) & 1023) - oz;
-          int src = args.zero_node;
-          if (sx >= 0 && sy >= 0 && sz >= 0 && sx < side && sy < side && sz < side)
-            src = level_offset_d(level) + static_cast<int>(morton3(sx, sy, sz)) - args.node_base;
-          const size_t goff = static_cast<size_t>(src) * args.box_bytes +
-                              static_cast<size_t>(kc) * static_cast<size_t>(args.Kp * kKChunk * 2);
-          const uint32_t soff = static_cast<uint32_t>(h) * a_bytes + static_cast<uint32_t>(m) * a_tile +
-                                static_cast<uint32_t>(t - m * T) * box_chunk;
-          bulk_g2s(st + soff, (h ? args.a_lo : args.a_hi) + goff, box_chunk, &full[s]);
-        } else {
-          const int h = c - n_a;
-          const uint8_t *bsrc = args.b_tiles + (static_cast<size_t>(slot) * nkc + kc) * 2u * btile + h * btile;
-          // B_lo right after B_hi (both kcw wide): the 2 Npad rows form one
-          // operand of uniform row-group stride for the fused-N MMA
-          const uint32_t bw = static_cast<uint32_t>(args.Npad) * kcw * 2u;
-          bulk_g2s(st + 2 * a_bytes + h * bw, bsrc, bw, &full[s]);
+        uint8_t *st = smem + static_cast<uint32_t>(s) * stage_bytes;
+        if (lane == 0) {
+          mbar_expect_tx(&full[s], bytes);
+          if (rows)
+            tc::tma_load_4d(st, map, alpha, x, y, z, &full[s]);
+          else
+            bulk_g2s(st + kABytes, tile, bytes, &full[s]);
+          (rows ? last_a : last_b)[s] = i;
+        }
+        alpha += 2 * kChunk;
+        tile += bytes;
+        if (++s == S) {
+          s = 0;
+          phase ^= 1u;
         }
       }
-      __syncwarp();
-      if (lane == 0) atomicMax(&last_unit[s], u);
     }
-  } else if (tid == 0) {
-    // MMA issuer: waits for each unit's operands, issues its MMAs, commits
-    // to the unit's empty barrier (arrives when those MMAs completed).  The
-    // shared-memory descriptors are built once: a byte offset o < 256 KB is
-    // added to a descriptor as o >> 4 in its 14-bit start-address field.
-    const uint32_t idesc = instr_desc_bf16(args.Npad);
-    const uint32_t idesc2 = instr_desc_bf16(2 * args.Npad); // fused: N = [B_hi | B_lo]
-    const bool fuse = args.fuse_n != 0;
-    const uint64_t desc_full = smem_desc(smem_u32(stage0), 128u, kKChunk * 16u); // SBO = chunk width * 16 B
-    const uint64_t desc_half = smem_desc(smem_u32(stage0), 128u, 16u * 16u);     // last chunk 16 wide
-    const uint64_t o_alo = a_bytes >> 4, o_bhi = (2u * a_bytes) >> 4;
+  } else if (warp == 0) {
+    // MMA issuer.  A: K-major rows of 64 bytes, 64-byte swizzle (hi in the
+    // first half, lo in the second); B: K-major core matrices, no swizzle,
+    // lo rows after the hi rows.
+    const int cols = args.cols;
+    const int wide = args.fused ? 2 * cols : cols;
+    const int w1 = piece_width(wide), w2 = piece_width(cols); // (at most two pieces each)
+    const uint32_t i1a = instr_desc_bf16(w1), i1b = instr_desc_bf16(wide - w1);
+    const uint32_t i2a = instr_desc_bf16(w2), i2b = instr_desc_bf16(cols - w2);
+    const bool split1 = wide > w1, split2 = cols > w2, fused = args.fused != 0;
+    const uint64_t da0 = tc::smem_desc_sw64(smem_u32(smem));
+    const uint64_t db0 = smem_desc(smem_u32(smem) + kABytes, 128u, 256u);
+    const uint64_t b_lo = (static_cast<uint32_t>(cols) * kChunk * 2u) >> 4;
     uint32_t accumulate = 0;
-    int issued = 0;
-    int s = 0, kc = 0;
+    int s = 0, issued = 0;
     uint32_t phase = 0;
-    for (int u = 0; u < units; ++u) {
-      if (!mbar_wait(&full[s], phase, args.wait_limit)) {
-        *abort_flag = 1;
-        atomicExch(args.error_flag, 2);
+    for (int i = 0; i < items; ++i) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&full[s], phase, args.wait_limit))) {
+        if (lane == 0) {
+          *abort_flag = 1;
+          atomicExch(args.error_flag, 2);
+        }
         break;
       }
       tc_fence_after();
-      const int kcw = min(kKChunk, args.Kpad - kc * kKChunk);
-      const uint64_t base = (kcw == kKChunk ? desc_full : desc_half) + ((static_cast<uint32_t>(s) * stage_bytes) >> 4);
-      const uint64_t o_blo = (2u * a_bytes + static_cast<uint32_t>(args.Npad) * kcw * 2u) >> 4;
-#pragma unroll
-      for (int ks = 0; ks < kKChunk / 16; ++ks) {
-        if (ks * 16 < kcw) {
-          const uint64_t o = base + static_cast<uint64_t>(ks * 16); // 2 core matrices = 256 B
-#pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            if (m < m_active) {
-              const uint32_t d = tmem + static_cast<uint32_t>(m * args.acc_stride);
-              const uint64_t ah = o + ((static_cast<uint32_t>(m) * a_tile) >> 4);
-              if (fuse) {
-                // columns [0, Npad): hi*hi + lo*hi; [Npad, 2 Npad): hi*lo
-                mma_bf16(d, ah, o + o_bhi, idesc2, accumulate);
-                mma_bf16(d, ah + o_alo, o + o_bhi, idesc, 1);
-              } else {
-                mma_bf16(d, ah, o + o_bhi, idesc, accumulate);
-                mma_bf16(d, ah, o + o_blo, idesc, 1);
-                mma_bf16(d, ah + o_alo, o + o_bhi, idesc, 1);
-              }
-            }
-          }
-          accumulate = 1;
+      if (lane == 0) {
+        const uint64_t off = (static_cast<uint32_t>(s) * stage_bytes) >> 4;
+        const uint64_t da = da0 + off, db = db0 + off;
+        const uint64_t db2 = db + static_cast<uint64_t>(w2) * 2;
+        // A_hi x B_hi (and, fused, x B_lo in its own columns)
+        mma_bf16(tmem, da, db, i1a, accumulate);
+        if (split1) mma_bf16(tmem + w1, da, db + static_cast<uint64_t>(w1) * 2, i1b, accumulate);
+        if (!fused) {
+          mma_bf16(tmem, da, db + b_lo, i2a, 1);
+          if (split2) mma_bf16(tmem + w2, da, db2 + b_lo, i2b, 1);
         }
+        mma_bf16(tmem, da + (kChunk * 2 >> 4), db, i2a, 1);
+        if (split2) mma_bf16(tmem + w2, da + (kChunk * 2 >> 4), db2, i2b, 1);
+        mma_commit(&empty[s]);
       }
-      mma_commit(&empty[s]);
-      issued = u + 1;
+      accumulate = 1;
+      issued = i + 1;
       if (++s == S) {
         s = 0;
         phase ^= 1u;
       }
-      if (++kc == nkc) kc = 0;
     }
     // The last commit arrives once every MMA issued before it has completed.
-    if (issued > 0 && !mbar_wait(&empty[(issued - 1) % S], ((issued - 1) / S) & 1)) {
-      *abort_flag = 1;
-      atomicExch(args.error_flag, 3);
+    if (issued > 0 && !__all_sync(0xffffffffu, mbar_wait(&empty[(issued - 1) % S], ((issued - 1) / S) & 1))) {
+      if (lane == 0) {
+        *abort_flag = 1;
+        atomicExch(args.error_flag, 3);
+      }
+    }
+  } else {
+    // parents of the tile (one per K rows): where their rows of R start
+    const int nx = lv.bx / K; // (used where whole parents fill a tile)
+    for (int q = lane; q < nx * lv.by * lv.bz; q += 32) {
+      const int px = x0 / K + q % nx, py = y0 + (q / nx) % lv.by, pz = z0 + q / (nx * lv.by);
+      seg_base[q] = (px < side && py < side && pz < side)
+                        ? ((level_box + 8LL * morton3(px, py, pz)) + group * (8 / args.groups)) * args.n_out * K
+                        : -1;
     }
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (*abort_flag != 0 && tid < S) {
-    // Abort: the copies of the last unit issued into each stage may still be
-    // in flight (earlier units of a stage completed before it was reused).
-    // Wait for them with the full limit before the CTA's shared memory is
-    // released.
-    const int u = last_unit[tid];
-    if (u >= 0) mbar_wait(&full[tid], static_cast<uint32_t>(u / S) & 1u);
+  const bool bad = *abort_flag != 0;
+  if (bad && tid < S) {
+    // Abort: the copies of the last chunk issued into each stage may still
+    // be in flight (earlier chunks of a stage completed before it was
+    // reused).  Wait for them with the full limit before the CTA's shared
+    // memory is reused or released.
+    const int i = max(last_a[tid], last_b[tid]);
+    if (i >= 0) mbar_wait(&full[tid], static_cast<uint32_t>(i / S) & 1u);
   }
+  if (bad) __syncthreads();
 
-  // Epilogue: warp w owns TMEM lanes 32w..32w+31 (rows of every M tile).
-  // A row's n_out reduced locals go to its column of the (now idle) stage
-  // memory at their full ranks, the other locals follow from the trace
-  // relations, and all n are scaled by D_L and stored.  After an expired
-  // wait the accumulators are incomplete: the tile's locals are written as
-  // NaN instead.
-  if (*abort_flag != 0) {
-    const int tr = tid / args.Kp;
-    const int k = tid - tr * args.Kp;
-    for (int m = 0; m < m_active; ++m) {
-      const int tt = m * T + tr;
-      if (tr < T && tt < count && k < args.K) {
-        const long long base = static_cast<long long>(tgt_node[tt]) * args.n * args.K + k;
-        for (int b = 0; b < args.n; ++b) {
-          if (args.L_list != nullptr)
-            args.L_list[k][static_cast<long long>(tgt_node[tt]) * args.n + b] = __int_as_float(0x7fc00000);
-          else
-            args.L[base + static_cast<long long>(b) * args.K] = __int_as_float(0x7fc00000);
-        }
-      }
+  // Epilogue: warp w owns TMEM lanes 32w..32w+31, one row per thread.  Column
+  // q of the group is local (class, beta) = (q / n_out, q % n_out), which is
+  // float q * K + state of the parent's rows of R.  Many states: consecutive
+  // lanes are consecutive states, stored directly; few: 32 columns at a time
+  // go through the idle stage memory, so that a warp stores the contiguous
+  // 32 K floats of one parent.
+  float *R = args.R + split * args.split_stride;
+  const int n_cols = (8 / args.groups) * args.n_out;
+  const uint32_t tlane = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+  auto load16 = [&](int c0, float (&v)[16]) {
+    tmem_ld16(tlane + static_cast<uint32_t>(c0), v);
+    if (args.fused) {
+      float w[16];
+      tmem_ld16(tlane + static_cast<uint32_t>(args.cols + c0), w);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] += w[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = bad ? __int_as_float(0x7fc00000) : items == 0 ? 0.0F : v[j];
+  };
+  if (K >= 32) {
+    const int rx = tid % lv.bx, ry = (tid / lv.bx) % lv.by, rz = tid / (lv.bx * lv.by);
+    const int px = (x0 + rx) / K, k = (x0 + rx) - px * K, py = y0 + ry, pz = z0 + rz;
+    const bool valid = rz < lv.bz && px < side && py < side && pz < side;
+    const long long base =
+        valid ? ((level_box + 8LL * morton3(px, py, pz)) + group * (8 / args.groups)) * args.n_out * K + k : 0;
+    for (int c0 = 0; c0 < args.cols; c0 += 16) {
+      float v[16];
+      load16(c0, v);
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (valid && c0 + j < n_cols) R[base + static_cast<long long>(c0 + j) * K] = v[j];
     }
   } else {
-    const int warp = tid >> 5;
-    const int row = tid;
-    const int tr = row / args.Kp;
-    const int k = row - tr * args.Kp;
-    const float *sl = args.scale_l + level * args.n;
-    float *const ep = reinterpret_cast<float *>(smem) + tid; // this row's locals, stride kTcThreads floats
-    for (int m = 0; m < m_active; ++m) {
-      const int tt = m * T + tr;
-      const bool valid = tr < T && tt < count && k < args.K;
-      const int node = valid ? tgt_node[tt] : 0;
-      const long long base = static_cast<long long>(node) * args.n * args.K + k;
-      float *const out_k = (args.L_list != nullptr && valid) ? args.L_list[k] + static_cast<long long>(node) * args.n
-                                                              : nullptr;
-      for (int c0 = 0; c0 < args.Npad; c0 += 16) {
+    float *slab = reinterpret_cast<float *>(smem);
+    const int segs = (lv.bx / K) * lv.by * lv.bz;
+    const uint32_t magic = 65536u / static_cast<uint32_t>(K) + 1u; // e / K = e * magic >> 16 for e < 1024, K < 32
+    for (int c0 = 0; c0 < args.cols; c0 += kSlab) {
+      for (int h = 0; h < kSlab && c0 + h < args.cols; h += 16) {
         float v[16];
-        const uint32_t tcol = tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(m * args.acc_stride + c0);
-        tmem_ld16(tcol, v);
-        if (args.fuse_n) {
-          float w[16];
-          tmem_ld16(tcol + static_cast<uint32_t>(args.Npad), w);
+        load16(c0 + h, v);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] += w[j];
-        }
-        if (units == 0) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = 0.0F; // no source box in the grid: no MMA wrote the accumulator
-        }
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (c0 + j < args.n_out) ep[__ldg(args.expand + c0 + j) * kTcThreads] = v[j];
+        for (int j = 0; j < 16; ++j) slab[tid * kSlabPitch + h + j] = v[j];
       }
-      for (int i = 0; i < args.n_derived; ++i) {
-        const int e = __ldg(args.expand + args.n_out + i);
-        ep[(e & 1023) * kTcThreads] = -(ep[((e >> 10) & 1023) * kTcThreads] + ep[(e >> 20) * kTcThreads]);
-      }
-      if (valid) {
-        for (int b = 0; b < args.n; ++b) {
-          const float x = ep[b * kTcThreads] * sl[b];
-          if (out_k != nullptr)
-            out_k[b] = x;
-          else
-            args.L[base + static_cast<long long>(b) * args.K] = x;
+      __syncthreads();
+      const int run = min(kSlab, n_cols - c0) * K;
+      for (int q = warp; q < segs; q += kTcThreads / 32) {
+        const long long base = seg_base[q];
+        if (base < 0) continue;
+        float *dst = R + base + static_cast<long long>(c0) * K;
+        for (int e = lane; e < run; e += 32) {
+          const int c = static_cast<int>((static_cast<uint32_t>(e) * magic) >> 16);
+          dst[e] = slab[(q * K + e - c * K) * kSlabPitch + c];
         }
       }
+      __syncthreads();
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (tid < 32) {
+  if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(args.tmem_cols));
+    tc::tmem_dealloc(tmem, args.tmem_cols);
   }
 }
 
-// Pack: scaled multipoles of levels 2..depth -> BF16 hi/lo boxes.  A box is
-// Kp rows (states) x Kpad alphas stored chunk by chunk (32 alphas; the last
-// chunk may be 16), each chunk as [Kp/8 row groups][w/8 column blocks][8][8]
-// so one box's rows of one chunk are contiguous.  One extra all-zero box
-// (index n_boxes) stands for sources outside the grid.  One CTA per box: a
-// chunk's 32 alphas x Kp states are read along the states (coalesced rows
-// of M[node][alpha][k]) into a shared tile, then written as 16-byte runs of
-// 8 alphas (one core-matrix row of hi and of lo).
+// Sum of the splits' reduced locals into the first split's, in a fixed order:
+// a CTA takes 32 float4 positions, its 8 groups of threads every eighth split
+// (the splits of one position are all the loads there are when the tree is
+// small).
+constexpr int kSumItems = 32, kSumGroups = 8;
+
+__global__ void __launch_bounds__(kSumItems * kSumGroups) m2l_sum_splits_kernel(float4 *__restrict__ R, long long vec,
+                                                                                int splits) {
+  __shared__ float4 part[kSumGroups][kSumItems];
+  const int item = threadIdx.x % kSumItems, group = threadIdx.x / kSumItems;
+  const long long at = static_cast<long long>(blockIdx.x) * kSumItems + item;
+  float4 v = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+  if (at < vec) {
+#pragma unroll 4
+    for (int s = group; s < splits; s += kSumGroups) {
+      const float4 x = R[at + s * vec];
+      v.x += x.x;
+      v.y += x.y;
+      v.z += x.z;
+      v.w += x.w;
+    }
+  }
+  part[group][item] = v;
+  __syncthreads();
+  if (group == 0 && at < vec) {
+    for (int g = 1; g < kSumGroups; ++g) {
+      const float4 x = part[g][item];
+      v.x += x.x;
+      v.y += x.y;
+      v.z += x.z;
+      v.w += x.w;
+    }
+    R[at] = v;
+  }
+}
+
+// Pack: multipoles of levels 2..depth, folded, scaled and split into BF16
+// hi / lo, as rows of the M2L operand: level by level,
+// [parent z][parent y][parent x][state][child class][16-alpha chunk][hi 16 | lo 16].
+// A CTA takes 8 (parent, state) columns with their 8 children: one parent and
+// 8 states where K >= 8, else as many whole parents as fit; it reads the
+// children's coefficients in runs of states into shared memory and writes a
+// parent's rows of those states as one contiguous run.
+// Bound: HBM (4 n bytes read and 4 (p+1)^2 written per box and state).
 constexpr int kPackThreads = 256;
-constexpr int kPackMaxKp = 128;
+constexpr int kPackCols = 64; // (parent, state, child)
+constexpr int kPackPitch = kPackCols + 1;
 
 __global__ void __launch_bounds__(kPackThreads) m2l_pack_kernel(const float *__restrict__ M,
                                                                 const float *const *__restrict__ M_list,
-                                                                const float *__restrict__ scale_m,
                                                                 const int *__restrict__ fold_off,
-                                                                const int *__restrict__ fold, int n_in,
-                                                                uint4 *__restrict__ hi, uint4 *__restrict__ lo, int n,
-                                                                int K, int Kp, int Kpad, int depth, int node_base,
-                                                                int n_boxes) {
-  __shared__ float tile[kKChunk][kPackMaxKp + 1]; // [alpha in chunk][state]
-  const int box = blockIdx.x;
+                                                                const int *__restrict__ fold, int n_fold, int n_in,
+                                                                uint4 *__restrict__ out, int n, int K, int chunks,
+                                                                int depth, int nP) {
+  extern __shared__ uint4 pack_smem[];
+  const int row_vec = chunks * 4;                    // 16-byte vectors of an operand row
+  const int row_pitch = (row_vec + 1) * 4;           // words of a staged row (one vector of padding)
+  uint32_t *rows = reinterpret_cast<uint32_t *>(pack_smem);       // [kPackCols][row_pitch]
+  float *sM = reinterpret_cast<float *>(rows + kPackCols * row_pitch); // [n][kPackPitch]
+  float *coef = sM + n * kPackPitch;                 // [n_fold] scaled fold coefficients
+  int *from = reinterpret_cast<int *>(coef + n_fold); // [n_fold] sM rows
+  int *off = from + n_fold;                          // [n_in + 1]
   const int tid = threadIdx.x;
-  const int node = node_base + box;
-  int level = 0;
-  while (level < depth && level_offset_d(level + 1) <= node) ++level;
-  const float *src = M != nullptr ? M + static_cast<long long>(node) * n * K : nullptr;
-  const long long box_vec = static_cast<long long>(box) * Kp * Kpad / 8; // 16-byte vectors before this box
-  const int nkc = (Kpad + kKChunk - 1) / kKChunk;
-  for (int kc = 0; kc < nkc; ++kc) {
-    const int w = min(kKChunk, Kpad - kc * kKChunk);
-    const int ncj = w / 8;
-    __syncthreads();
-    for (int e = tid; e < w * Kp; e += kPackThreads) {
-      const int al = e / Kp;
-      const int k = e - al * Kp;
-      const int j = kc * kKChunk + al;
-      // folded input j: sum of c M_a over its fold entries (all of one
-      // degree, the first one its own rank), then scaled (scale_m is one
-      // power of two per degree).  Padding inputs (j >= n_in), padding
-      // states (k >= K) and the zero box are zero.
-      float m = 0.0F;
-      if (box < n_boxes && j < n_in && k < K) {
-        const int f0 = __ldg(fold_off + j), f1 = __ldg(fold_off + j + 1);
-        for (int f = f0; f < f1; ++f) {
-          const int ent = __ldg(fold + f);
-          const int a = ent & 0xffff;
-          const float x =
-              M_list != nullptr ? M_list[k][static_cast<long long>(node) * n + a] : src[static_cast<long long>(a) * K + k];
-          m = fmaf(static_cast<float>((ent >> 16) - 64), x, m);
-        }
-        m *= scale_m[level * n + (__ldg(fold + f0) & 0xffff)];
-      }
-      tile[al][k] = m;
+  const int kblocks = (K + 7) / 8;
+  const int k0 = (blockIdx.x % kblocks) * 8;
+  const int kc = min(8, K - k0);
+  const int parent0 = 1 + (blockIdx.x / kblocks) * nP; // node index of the first parent (levels 1..depth - 1)
+  int level = 2;
+  while (level_offset_d(level) <= parent0) ++level; // the children's level
+  const int cols = nP * kc * 8;            // column = (parent, state, child)
+  const long long child0 = 8LL * parent0 + 1;
+  if (M_list != nullptr) {
+    for (int e = tid; e < kc * 8 * n; e += kPackThreads) {
+      const int k = e / (8 * n), r = e - k * 8 * n;
+      const int c = r / n, a = r - c * n;
+      for (int q = 0; q < nP; ++q)
+        sM[a * kPackPitch + (q * kc + k) * 8 + c] = M_list[k0 + k][(child0 + 8 * q) * n + r];
     }
-    __syncthreads();
-    const long long chunk_vec = box_vec + static_cast<long long>(kc) * Kp * kKChunk / 8;
-    for (int v = tid; v < Kp * w / 8; v += kPackThreads) {
-      const int x = v >> 3;
-      const int r8 = v & 7;
-      const int cjl = x % ncj;
-      const int k = (x / ncj) * 8 + r8;
-      uint32_t h[4], l[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float v0 = tile[cjl * 8 + 2 * j][k], v1 = tile[cjl * 8 + 2 * j + 1][k];
-        const __nv_bfloat16 h0 = __float2bfloat16_rn(v0), h1 = __float2bfloat16_rn(v1);
-        const __nv_bfloat16 l0 = __float2bfloat16_rn(v0 - __bfloat162float(h0));
-        const __nv_bfloat16 l1 = __float2bfloat16_rn(v1 - __bfloat162float(h1));
-        h[j] = static_cast<uint32_t>(__bfloat16_as_ushort(h0)) | (static_cast<uint32_t>(__bfloat16_as_ushort(h1)) << 16);
-        l[j] = static_cast<uint32_t>(__bfloat16_as_ushort(l0)) | (static_cast<uint32_t>(__bfloat16_as_ushort(l1)) << 16);
-      }
-      hi[chunk_vec + v] = make_uint4(h[0], h[1], h[2], h[3]);
-      lo[chunk_vec + v] = make_uint4(l[0], l[1], l[2], l[3]);
+  } else if ((K & 3) == 0) {
+    const int quads = kc >> 2;
+    for (int e = tid; e < nP * 8 * n * quads; e += kPackThreads) {
+      const int kq = e % quads, t = e / quads;
+      const int a = t % n, b = t / n; // box b of the CTA
+      const float4 v = *reinterpret_cast<const float4 *>(M + ((child0 + b) * n + a) * K + k0 + 4 * kq);
+      float *dst = sM + a * kPackPitch + ((b >> 3) * kc + 4 * kq) * 8 + (b & 7);
+      dst[0] = v.x;
+      dst[8] = v.y;
+      dst[16] = v.z;
+      dst[24] = v.w;
+    }
+  } else {
+    for (int e = tid; e < nP * 8 * n * kc; e += kPackThreads) {
+      const int k = e % kc, t = e / kc;
+      const int a = t % n, b = t / n;
+      sM[a * kPackPitch + ((b >> 3) * kc + k) * 8 + (b & 7)] = M[((child0 + b) * n + a) * K + k0 + k];
     }
   }
+  for (int e = tid; e <= n_in; e += kPackThreads) off[e] = __ldg(fold_off + e);
+  for (int e = tid; e < n_fold; e += kPackThreads) {
+    // the entries of one input are of one degree: its scaling 2^(level degree) is exact
+    const int ent = __ldg(fold + e);
+    const int a = ent & 0xffff;
+    int deg = 0;
+    while (basis_size_d(deg) <= a) ++deg;
+    from[e] = a * kPackPitch;
+    coef[e] = static_cast<float>((ent >> 16) - 64) * __int_as_float((127 + level * deg) << 23);
+  }
+  __syncthreads();
+  // pairs of inputs: two folded moments, their hi and lo halves as one word each
+  for (int e = tid; e < chunks * 8 * kPackCols; e += kPackThreads) {
+    const int col = e & (kPackCols - 1), jp = e / kPackCols;
+    if (col >= cols) continue;
+    float m[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = 2 * jp + h;
+      m[h] = 0.0F;
+      if (j < n_in)
+        for (int f = off[j]; f < off[j + 1]; ++f) m[h] = fmaf(coef[f], sM[from[f] + col], m[h]);
+    }
+    const __nv_bfloat16 h0 = __float2bfloat16_rn(m[0]), h1 = __float2bfloat16_rn(m[1]);
+    const __nv_bfloat16 l0 = __float2bfloat16_rn(m[0] - __bfloat162float(h0));
+    const __nv_bfloat16 l1 = __float2bfloat16_rn(m[1] - __bfloat162float(h1));
+    uint32_t *row = rows + col * row_pitch + (jp >> 3) * 16 + (jp & 7);
+    row[0] = static_cast<uint32_t>(__bfloat16_as_ushort(h0)) | (static_cast<uint32_t>(__bfloat16_as_ushort(h1)) << 16);
+    row[8] = static_cast<uint32_t>(__bfloat16_as_ushort(l0)) | (static_cast<uint32_t>(__bfloat16_as_ushort(l1)) << 16);
+  }
+  __syncthreads();
+  const long long level_row = static_cast<long long>(level_offset_d(level) - level_offset_d(2)) * K;
+  const int side = 1 << (level - 1);
+  for (int q = 0; q < nP; ++q) {
+    int px, py, pz;
+    demorton3(static_cast<uint32_t>(parent0 + q - level_offset_d(level - 1)), px, py, pz);
+    const long long row0 = level_row + ((static_cast<long long>(pz * side + py) * side + px) * K + k0) * 8;
+    const int run = kc * 8 * row_vec;
+    for (int e = tid; e < run; e += kPackThreads)
+      out[row0 * row_vec + e] =
+          *reinterpret_cast<const uint4 *>(rows + (q * kc * 8 + e / row_vec) * row_pitch + (e % row_vec) * 4);
+  }
+}
+
+// Operator tiles: [27 neighbours][8 source classes][group][chunk][hi, lo] of
+// cols rows (class, beta) x 16 alphas in K-major core matrices
+// [cols / 8][2][8][8], from the FP64 derivatives deriv[343][ranks of degree
+// <= 2p] (zero in touching slots, which also zeroes the parent itself).
+__global__ void __launch_bounds__(256) m2l_operator_kernel(const double *__restrict__ deriv, int n_deriv, int p,
+                                                           int groups, int cols, int chunks,
+                                                           __nv_bfloat16 *__restrict__ out) {
+  int t = blockIdx.x;
+  const int chunk = t % chunks;
+  t /= chunks;
+  const int group = t % groups;
+  t /= groups;
+  const int cs = t & 7, sh = t >> 3;
+  const int n_out = (p + 1) * (p + 1), per = 8 / groups;
+  // exponents of reduced output i (ascending ranks with z <= 1): degree d
+  // starts at d^2; per x: (x, d - x - 1, 1) then (x, d - x, 0)
+  auto exponents = [](int i, int &x, int &y, int &z) {
+    int d = 0;
+    while ((d + 1) * (d + 1) <= i) ++d;
+    const int r = i - d * d;
+    x = r >> 1;
+    z = (r == 2 * d) ? 0 : 1 - (r & 1);
+    y = d - x - z;
+  };
+  __nv_bfloat16 *hi = out + static_cast<size_t>(blockIdx.x) * 2 * cols * kChunk;
+  __nv_bfloat16 *lo = hi + static_cast<size_t>(cols) * kChunk;
+  for (int e = threadIdx.x; e < cols * kChunk; e += blockDim.x) {
+    const int al = e % kChunk, col = e / kChunk;
+    const int alpha = chunk * kChunk + al + 1; // reduced inputs are the outputs without rank 0
+    double v = 0.0;
+    if (col < per * n_out && alpha < n_out) {
+      const int cl = group * per + col / n_out;
+      int ax, ay, az, bx, by, bz;
+      exponents(alpha, ax, ay, az);
+      exponents(col % n_out, bx, by, bz);
+      const int ox = (cl & 1) - (cs & 1) - 2 * (sh % 3 - 1), oy = ((cl >> 1) & 1) - ((cs >> 1) & 1) - 2 * ((sh / 3) % 3 - 1),
+                oz = ((cl >> 2) & 1) - ((cs >> 2) & 1) - 2 * (sh / 9 - 1);
+      const int slot = (ox + 3) * 49 + (oy + 3) * 7 + (oz + 3);
+      v = deriv[static_cast<size_t>(slot) * n_deriv + rank3(ax + bx, ay + by, az + bz)];
+    }
+    const __nv_bfloat16 h = __float2bfloat16_rn(static_cast<float>(v));
+    const int at = ((col / 8) * 2 + al / 8) * 64 + (col % 8) * 8 + al % 8;
+    hi[at] = h;
+    lo[at] = __float2bfloat16_rn(static_cast<float>(v - static_cast<double>(__bfloat162float(h))));
+  }
+}
+
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// The driver's tensor-map encoder, looked up at run time (the library links
+// the CUDA runtime only).
+EncodeTiled encode_tiled() {
+  static const EncodeTiled fn = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return reinterpret_cast<EncodeTiled>(p);
+  }();
+  return fn;
 }
 
 } // namespace
 
-size_t m2l_tc_smem_bytes(int Npad, int m_tiles, int stages, int n) {
-  const size_t a = 128u * kKChunk * 2u * static_cast<size_t>(m_tiles);
-  const size_t b = static_cast<size_t>(Npad) * kKChunk * 2u;
-  const size_t epi = (static_cast<size_t>(kTcThreads) * n * 4u + 15u) & ~static_cast<size_t>(15);
-  return std::max(static_cast<size_t>(stages) * (2 * a + 2 * b), epi) + 2 * stages * sizeof(uint64_t) + 8 +
-         (2 * kTcMaxTargets + 216 + 1 + 8) * sizeof(int);
+M2lColumns m2l_columns(int p, bool fused) {
+  const int n_out = (p + 1) * (p + 1);
+  M2lColumns c;
+  c.chunks = std::max(1, (n_out - 1 + kChunk - 1) / kChunk);
+  for (c.groups = 1; c.groups <= 8; c.groups *= 2) {
+    c.cols = round_up(8 / c.groups * n_out, 16);
+    if ((fused ? 2 : 1) * c.cols <= 512) break;
+  }
+  return c;
 }
 
-void launch_m2l_pack(const float *M, const float *scale_m, const int *fold_off, const int *fold, int n_in, void *hi,
-                     void *lo, int n, int K, int Kp, int Kpad, int depth, int node_base, int n_boxes, cudaStream_t s,
-                     const float *const *M_list) {
-  if (Kp > kPackMaxKp || Kp % 8 != 0 || Kpad % 16 != 0) return; // the plan keeps Kp <= 128, multiples of 8
-  m2l_pack_kernel<<<n_boxes + 1, kPackThreads, 0, s>>>(M, M_list, scale_m, fold_off, fold, n_in,
-                                                        static_cast<uint4 *>(hi), static_cast<uint4 *>(lo), n, K, Kp,
-                                                        Kpad, depth, node_base, n_boxes);
+// Row boxes: K >= 32 states fill the rows along (x, state); fewer take whole
+// parents, in the box of at most 128 rows that covers the level in the fewest
+// tiles.  Splits: the count that minimises waves x (the split's tensor-core
+// cycles + a CTA's fixed cost) + the cost of writing and summing the partial
+// locals, in SM cycles (fixed cost about 9,000, 6,000 for the summing kernel;
+// partial sums at 3 TB/s).
+M2lGrid m2l_grid(int depth, int K, const M2lColumns &c, int n_out, int sm_count, int max_splits) {
+  M2lGrid g;
+  double boxes = 0.0;
+  for (int level = 2; level <= depth; ++level) {
+    M2lLevel &l = g.levels[level - 2];
+    const int P = 1 << (level - 1);
+    l.side = P;
+    if (K >= 32) {
+      l.bx = std::min(kM2lRows, P * K);
+      l.by = std::min(P, kM2lRows / l.bx);
+      l.bz = std::min(P, kM2lRows / (l.bx * l.by));
+    } else {
+      long long best = -1;
+      for (int nx = 1; nx <= P && nx * K <= kM2lRows; ++nx)
+        for (int ny = 1; ny <= P && nx * ny * K <= kM2lRows; ++ny) {
+          const int nz = std::min(P, kM2lRows / (nx * ny * K));
+          const auto ceil_div = [](int a, int b) { return static_cast<long long>((a + b - 1) / b); };
+          const long long tiles = ceil_div(P, nx) * ceil_div(P, ny) * ceil_div(P, nz);
+          // fewest tiles; among those the box with the fewest rows (less to load)
+          const long long cost = tiles * 1024 + nx * ny * nz * K;
+          if (best < 0 || cost < best) {
+            best = cost;
+            l.bx = nx * K;
+            l.by = ny;
+            l.bz = nz;
+          }
+        }
+    }
+    l.tx = (P * K + l.bx - 1) / l.bx;
+    l.ty = (P + l.by - 1) / l.by;
+    l.tz = (P + l.bz - 1) / l.bz;
+    g.tiles += l.tx * l.ty * l.tz;
+    boxes += static_cast<double>(P) * P * P * 8.0;
+  }
+  const int pairs = 26 * 8;
+  const double pair_cycles = c.chunks * 3.0 * c.cols / 2.0;
+  const double partial = boxes * n_out * K * 8.0 / 3e12 * 1.9e9;
+  double best = 0.0;
+  for (int s = 1; s <= std::min(max_splits, kM2lMaxSplits); ++s) {
+    const long long ctas = static_cast<long long>(g.tiles) * c.groups * s;
+    const double waves = static_cast<double>((ctas + sm_count - 1) / sm_count);
+    const double cost =
+        waves * (((pairs + s - 1) / s) * pair_cycles + 9000.0) + (s > 1 ? 6000.0 + s * partial : 0.0);
+    if (s == 1 || cost < best) {
+      best = cost;
+      g.splits = s;
+    }
+  }
+  return g;
 }
 
-void launch_m2l_tc(const TcArgs &args, int n_tiles, cudaStream_t s) {
-  if (n_tiles == 0) return;
-  size_t smem = m2l_tc_smem_bytes(args.Npad, args.m_tiles, args.stages, args.n);
+size_t m2l_operand_bytes(int depth, int K, int chunks) {
+  return static_cast<size_t>(level_offset_d(depth + 1) - level_offset_d(2)) * K * chunks * kChunk * 4;
+}
+
+bool m2l_set_operand(M2lTcArgs &args, const M2lGrid &grid, void *a) {
+  const EncodeTiled encode = encode_tiled();
+  if (encode == nullptr) return false;
+  args.tiles = grid.tiles;
+  args.splits = grid.splits;
+  const size_t row = static_cast<size_t>(args.chunks) * kChunk * 4; // bytes of one (state, class) row
+  for (int level = 2; level <= args.depth; ++level) {
+    const M2lLevel &l = grid.levels[level - 2];
+    args.levels[level - 2] = l;
+    uint8_t *base = static_cast<uint8_t *>(a) + static_cast<size_t>(level_offset_d(level) - level_offset_d(2)) * args.K * row;
+    const cuuint64_t xk = static_cast<cuuint64_t>(l.side) * args.K;
+    const cuuint64_t dims[4] = {static_cast<cuuint64_t>(args.chunks) * kChunk * 2 * 8, xk,
+                                static_cast<cuuint64_t>(l.side), static_cast<cuuint64_t>(l.side)};
+    const cuuint64_t strides[3] = {row * 8, row * 8 * xk, row * 8 * xk * l.side};
+    const cuuint32_t box[4] = {kChunk * 2, static_cast<cuuint32_t>(l.bx), static_cast<cuuint32_t>(l.by),
+                               static_cast<cuuint32_t>(l.bz)};
+    const cuuint32_t step[4] = {1, 1, 1, 1};
+    if (encode(&args.maps[level - 2], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base, dims, strides, box, step,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return false;
+  }
+  return true;
+}
+
+M2lOperator::~M2lOperator() {
+  if (b != nullptr) cudaFree(b);
+}
+
+std::shared_ptr<const M2lOperator> m2l_operator(int device, int p, const M2lColumns &c,
+                                                const std::vector<double> &T64) {
+  static std::mutex mutex;
+  static std::map<std::tuple<int, int, int>, std::weak_ptr<const M2lOperator>> cache;
+  std::lock_guard<std::mutex> lock(mutex);
+  std::weak_ptr<const M2lOperator> &slot = cache[std::make_tuple(device, p, c.groups)];
+  if (std::shared_ptr<const M2lOperator> have = slot.lock()) return have;
+  const int n = basis_size_d(p), n2 = basis_size_d(2 * p);
+  // derivatives of degree <= 2p: T[alpha][beta] depends on alpha + beta only
+  std::vector<double> deriv(static_cast<size_t>(343) * n2, 0.0);
+  std::vector<int> pick(static_cast<size_t>(n2), -1);
+  for (int d = 0; d <= 2 * p; ++d)
+    for (int x = 0; x <= d; ++x)
+      for (int y = 0; x + y <= d; ++y) {
+        const int z = d - x - y;
+        // any split into two multi-indices of degree <= p
+        int ax = std::min(x, p), ay = std::min(y, p - ax), az = std::min(z, p - ax - ay);
+        pick[static_cast<size_t>(rank3(x, y, z))] = rank3(ax, ay, az) * n + rank3(x - ax, y - ay, z - az);
+      }
+  for (size_t slot_i = 0; slot_i < 343; ++slot_i)
+    for (size_t r = 0; r < static_cast<size_t>(n2); ++r)
+      deriv[slot_i * n2 + r] = T64[slot_i * n * n + static_cast<size_t>(pick[r])];
+  auto op = std::make_shared<M2lOperator>();
+  op->device = device;
+  const int tiles = kM2lShifts * 8 * c.groups * c.chunks;
+  op->bytes = static_cast<size_t>(tiles) * b_tile_bytes(c.cols);
+  double *d = nullptr;
+  cudaError_t e = cudaMalloc(&op->b, op->bytes);
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&d), deriv.size() * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemcpy(d, deriv.data(), deriv.size() * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    m2l_operator_kernel<<<tiles, 256>>>(d, n2, p, c.groups, c.cols, c.chunks, static_cast<__nv_bfloat16 *>(op->b));
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+  if (d != nullptr) cudaFree(d);
+  if (e == cudaErrorMemoryAllocation) throw std::bad_alloc();
+  if (e != cudaSuccess) throw std::runtime_error(std::string("M2L operator tiles: ") + cudaGetErrorString(e));
+  slot = op;
+  return op;
+}
+
+size_t m2l_tc_smem_bytes(int cols, int stages) {
+  return std::max(static_cast<size_t>(stages) * stage_bytes_of(cols), sizeof(float) * kM2lRows * kSlabPitch) +
+         2 * kM2lMaxStages * sizeof(uint64_t) + kM2lRows * sizeof(long long) + 8 +
+         (1 + kM2lShifts + 2 * kM2lMaxStages) * sizeof(int);
+}
+
+static size_t pack_smem_bytes(int n, int n_fold, int n_in, int chunks) {
+  return static_cast<size_t>(kPackCols) * (chunks * 4 + 1) * 16 + sizeof(float) * n * kPackPitch +
+         (sizeof(float) + sizeof(int)) * static_cast<size_t>(n_fold) + sizeof(int) * (static_cast<size_t>(n_in) + 1);
+}
+
+void launch_m2l_pack(const float *M, const int *fold_off, const int *fold, int n_fold, int n_in, void *a, int n, int K,
+                     int chunks, int depth, cudaStream_t s, const float *const *M_list) {
+  const int nP = K >= 8 ? 1 : 8 / K; // divides 8, so a CTA's parents are of one level (K = 3: 2, K = 5..7: 1)
+  const int parents = level_offset_d(depth) - 1;
+  m2l_pack_kernel<<<(K + 7) / 8 * (parents / nP), kPackThreads, pack_smem_bytes(n, n_fold, n_in, chunks), s>>>(
+      M, M_list, fold_off, fold, n_fold, n_in, static_cast<uint4 *>(a), n, K, chunks, depth, nP);
+}
+
+int launch_m2l_tc(const M2lTcArgs &args, cudaStream_t s) {
+  size_t smem = m2l_tc_smem_bytes(args.cols, args.stages);
   // More than half of TMEM per CTA: request enough shared memory that a
   // second CTA never shares the SM (its tcgen05.alloc would wait for ours).
   if (args.tmem_cols > 256) smem = std::max<size_t>(smem, 120 * 1024);
-  if (args.m_tiles == 4)
-    m2l_tc_kernel<4><<<n_tiles, kTcThreads, smem, s>>>(args);
-  else if (args.m_tiles == 2)
-    m2l_tc_kernel<2><<<n_tiles, kTcThreads, smem, s>>>(args);
-  else
-    m2l_tc_kernel<1><<<n_tiles, kTcThreads, smem, s>>>(args);
+  m2l_tc_kernel<<<args.tiles * args.groups * args.splits, kTcThreads, smem, s>>>(args);
+  if (args.splits == 1) return 1;
+  const long long vec = args.split_stride / 4; // a multiple of 64 boxes
+  m2l_sum_splits_kernel<<<static_cast<unsigned>((vec + kSumItems - 1) / kSumItems), kSumItems * kSumGroups, 0, s>>>(
+      reinterpret_cast<float4 *>(args.R), vec, args.splits);
+  return 2;
 }
 
 // Self-test of the bounded-wait path: one thread waits on an mbarrier whose
@@ -508,47 +763,9 @@ void launch_bounded_wait_selftest(int *error_flag, cudaStream_t s) {
 }
 
 bool configure_m2l_tc(size_t max_smem) {
-  prefer_max_shared_carveout(m2l_tc_kernel<1>);
-  prefer_max_shared_carveout(m2l_tc_kernel<2>);
-  prefer_max_shared_carveout(m2l_tc_kernel<4>);
-  return allow_dynamic_smem(m2l_tc_kernel<1>, max_smem) && allow_dynamic_smem(m2l_tc_kernel<2>, max_smem) &&
-         allow_dynamic_smem(m2l_tc_kernel<4>, max_smem);
-}
-
-// Host: B tiles [slot][alpha chunk][hi, lo][Npad x 32 stride] BF16 from FP64
-// matrices T[slot][alpha][beta] (symmetric in alpha, beta); a chunk of width w
-// is stored as [beta group][w/8 column blocks][8 betas][8 alphas].
-std::vector<uint16_t> pack_m2l_b_tiles(const std::vector<double> &T64, int n, const M2lTraceless &red, int Npad,
-                                       int Kpad) {
-  const int nkc = (Kpad + kKChunk - 1) / kKChunk;
-  const size_t btile = static_cast<size_t>(Npad) * kKChunk;
-  std::vector<uint16_t> out(static_cast<size_t>(343) * nkc * 2 * btile, 0);
-  auto bf16_bits = [](float f) -> uint16_t {
-    const __nv_bfloat16 h = __float2bfloat16_rn(f);
-    uint16_t b;
-    std::memcpy(&b, &h, 2);
-    return b;
-  };
-  for (int slot = 0; slot < 343; ++slot) {
-    const double *Ts = T64.data() + static_cast<size_t>(slot) * n * n;
-    const int n_out = static_cast<int>(red.out_set.size()), n_in = static_cast<int>(red.in_set.size());
-    for (int beta = 0; beta < n_out; ++beta)
-      for (int alpha = 0; alpha < n_in; ++alpha) {
-        const double v = Ts[static_cast<size_t>(red.in_set[static_cast<size_t>(alpha)]) * n +
-                            red.out_set[static_cast<size_t>(beta)]];
-        const __nv_bfloat16 h = __float2bfloat16_rn(static_cast<float>(v));
-        const float l = static_cast<float>(v - static_cast<double>(__bfloat162float(h)));
-        const int kc = alpha / kKChunk;
-        const int al = alpha - kc * kKChunk;
-        const int ncj = std::min(kKChunk, Kpad - kc * kKChunk) / 8;
-        uint16_t *hi = out.data() + (static_cast<size_t>(slot) * nkc + kc) * 2 * btile;
-        uint16_t *lo = hi + btile;
-        const size_t at = ((static_cast<size_t>(beta / 8) * ncj + al / 8) * 8 + beta % 8) * 8 + al % 8;
-        hi[at] = bf16_bits(static_cast<float>(v));
-        lo[at] = bf16_bits(l);
-      }
-  }
-  return out;
+  prefer_max_shared_carveout(m2l_tc_kernel);
+  return encode_tiled() != nullptr && allow_dynamic_smem(m2l_tc_kernel, max_smem) &&
+         allow_dynamic_smem(m2l_pack_kernel, max_smem);
 }
 
 M2lTraceless m2l_traceless(int p) {

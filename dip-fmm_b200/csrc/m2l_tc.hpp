@@ -1,41 +1,69 @@
 // Tensor-core (tcgen05) M2L: launch interface.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
 #include <cstdint>
-#include <cstring>
+#include <memory>
 #include <vector>
+
+#include "far_kernels.hpp"
 
 namespace cdfmm_b200 {
 
-struct TcArgs {
-  const uint8_t *a_hi;     // packed BF16 hi boxes [box][32-alpha chunk][Kp/8][w/8][8][8] (folded moments)
-  const uint8_t *a_lo;     // packed BF16 lo boxes
-  const uint8_t *b_tiles;  // [343 slots][32-alpha chunk][hi, lo][Npad/8][w/8][8][8] (reduced operator)
-  const int4 *tiles;       // per CTA: (level, class, first parent Morton index, target count)
-  const float *scale_l;    // [depth+1][n] exact powers of two
-  float *L;                // [node][n][K] FP32 locals (overwritten)
-  float *const *L_list;    // or (stacked problems, one state each): state k's locals at L_list[k][node][n]
-  int *error_flag;         // set nonzero if a bounded wait expired
-  int n, K, Kp, Kpad, Npad;
-  int node_base;           // flat node index of packed box 0
-  int zero_node;           // packed index of the all-zero box
-  int stages;
-  int m_tiles;             // 128-row accumulators per CTA sharing each B tile
-  int acc_stride;          // TMEM columns between accumulators (multiple of 32)
-  int fuse_n;              // 1: A_hi x [B_hi | B_lo] as one N = 2 Npad MMA (acc_stride >= 2 Npad)
-  uint32_t tmem_cols;
-  uint32_t box_bytes;      // Kp * Kpad * 2
-  uint32_t wait_limit;     // iterations of each pipeline progress wait (kTcWaitLimit; 0 = expire at once)
-  // traceless reduction (M2lTraceless): accumulator column j holds the
-  // local of full rank expand[j] (j < n_out); expand[n_out + i] =
-  // d | s1 << 10 | s2 << 20 gives the remaining locals L_d = -(L_s1 + L_s2)
-  // in an order where both sources come first
-  const int *expand;
-  int n_out, n_derived;
+constexpr int kM2lMaxLevels = 7;  // tree levels 2..8
+constexpr int kM2lRows = 128;     // rows of one MMA tile
+constexpr int kM2lMaxStages = 8;
+constexpr int kM2lMaxSplits = 104; // two (neighbour, source class) pairs per CTA
+constexpr int kM2lShifts = 27;    // parent neighbours (the parent itself, index 13, has no list2 source)
+
+// Row tiles of one level: a tile is a box of bx consecutive (parent x,
+// state) rows times by x bz parents, at most 128 rows, tx x ty x tz of them.
+struct M2lLevel {
+  int side;       // parents per axis, 2^(level - 1)
+  int bx, by, bz;
+  int tx, ty, tz;
 };
+
+// Operator columns of an order: the 8 target classes in `groups` groups, each
+// `cols` accumulator columns (8 / groups classes x n_out locals, rounded up
+// to 16), and the 16-wide alpha chunks of the contraction.
+struct M2lColumns {
+  int groups = 1, cols = 16, chunks = 1;
+};
+M2lColumns m2l_columns(int p, bool fused);
+
+struct alignas(64) M2lTcArgs {
+  CUtensorMap maps[kM2lMaxLevels]; // operand of level l: maps[l - 2]
+  M2lLevel levels[kM2lMaxLevels];
+  const uint8_t *b;                // operator tiles (m2l_operator)
+  float *R;                        // [splits][box][n_out][K] reduced, unscaled locals (overwritten;
+                                   // the first split's then hold the sum)
+  long long split_stride;          // floats between splits
+  int *error_flag;                 // set nonzero if a bounded wait expired
+  int depth, K, n_out;
+  int groups, cols, chunks;
+  int splits;                      // CTAs sharing a tile's (parent neighbour, source class) sum
+  int tiles;
+  int stages;
+  int fused;                       // 1: A_hi x [B_hi | B_lo], the hi * lo product in its own columns
+  uint32_t tmem_cols;
+  uint32_t wait_limit;             // iterations of each pipeline progress wait (0 = expire at once)
+};
+
+// The reduced locals a launch with these arguments leaves in R.
+inline ReducedLocals reduced_locals(const M2lTcArgs &a, int k0 = 0) {
+  return {a.R, a.K, k0};
+}
+
+// Tile and split choice for K states on a tree of `depth` levels.
+struct M2lGrid {
+  M2lLevel levels[kM2lMaxLevels];
+  int tiles = 0, splits = 1;
+};
+M2lGrid m2l_grid(int depth, int K, const M2lColumns &c, int n_out, int sm_count, int max_splits);
 
 // Traceless reduction of the M2L (Cartesian Taylor basis of order p, n
 // coefficients).  The operator T[beta][alpha] = D^{alpha+beta} G with G
@@ -62,32 +90,36 @@ M2lTraceless m2l_traceless(int p);
 // Default iterations of a bounded mbarrier wait (about 2 s with the back-off).
 constexpr uint32_t kTcWaitLimit = 1u << 26;
 
-// Largest target count of one CTA: m_tiles (<= 4) x 128 / Kp with Kp >= 8.
-constexpr int kTcMaxTargets = 64;
+// Operator tiles of (device, order, groups) on the device, built there from
+// the FP64 derivative table of T64 ([343][n][n]) on first use and shared by
+// every plan that holds them; freed with the last of those.
+struct M2lOperator {
+  void *b = nullptr;
+  size_t bytes = 0;
+  int device = 0;
+  ~M2lOperator();
+};
+std::shared_ptr<const M2lOperator> m2l_operator(int device, int p, const M2lColumns &c,
+                                                const std::vector<double> &T64);
 
-// The reduction fields of a launch from the plan that owns the tables.
-template <class Plan> inline void set_m2l_reduction(TcArgs &ta, const Plan *p) {
-  ta.expand = p->tc_expand;
-  ta.n_out = p->tc_n_out;
-  ta.n_derived = p->tc_n_derived;
-}
+// Bytes of the packed operand of all boxes of levels 2..depth for K states.
+size_t m2l_operand_bytes(int depth, int K, int chunks);
+// Fills args.maps / levels / tiles / splits for the operand at `a`; false if
+// a tensor map cannot be encoded.
+bool m2l_set_operand(M2lTcArgs &args, const M2lGrid &grid, void *a);
 
-// Dynamic shared memory of the M2L kernel: the pipeline stages, or the
-// epilogue's 128 full-basis rows of n coefficients when larger.
-size_t m2l_tc_smem_bytes(int Npad, int m_tiles, int stages, int n);
-// Scaled, folded multipoles -> BF16 hi/lo boxes (fold_off / fold from
-// M2lTraceless, n_in reduced inputs, Kpad = 16 ceil(n_in / 16)).
-void launch_m2l_pack(const float *M, const float *scale_m, const int *fold_off, const int *fold, int n_in, void *hi,
-                     void *lo, int n, int K, int Kp, int Kpad, int depth, int node_base, int n_boxes, cudaStream_t s,
-                     const float *const *M_list = nullptr);
-void launch_m2l_tc(const TcArgs &args, int n_tiles, cudaStream_t s);
+// Dynamic shared memory of the M2L kernel.
+size_t m2l_tc_smem_bytes(int cols, int stages);
+// Scaled, folded multipoles -> BF16 hi/lo operand rows (fold_off / fold from
+// M2lTraceless).  M_list (stacked problems, one state each): state k's
+// multipoles at M_list[k][node][n]; else M[node][n][K].
+void launch_m2l_pack(const float *M, const int *fold_off, const int *fold, int n_fold, int n_in, void *a, int n, int K,
+                     int chunks, int depth, cudaStream_t s, const float *const *M_list = nullptr);
+// Returns the launch count (the sum over splits is a second kernel).
+int launch_m2l_tc(const M2lTcArgs &args, cudaStream_t s);
 bool configure_m2l_tc(size_t max_smem);
 // Runs a kernel whose bounded mbarrier wait must expire (nothing arrives)
 // and set *error_flag = 2, exactly as an expired wait of the M2L pipeline.
 void launch_bounded_wait_selftest(int *error_flag, cudaStream_t s);
-// B tiles of the reduced operator: element (beta row i, alpha column j) =
-// T[out_set[i]][in_set[j]] of the FP64 matrices T[slot][n][n].
-std::vector<uint16_t> pack_m2l_b_tiles(const std::vector<double> &T64, int n, const M2lTraceless &red, int Npad,
-                                       int Kpad);
 
 } // namespace cdfmm_b200

@@ -69,26 +69,6 @@ cudaError_t scratch_address(int device, void **out) {
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
-// Tensor-core M2L work tiles, written on the device (no host copy, no host
-// synchronisation): per level from `depth` down to 2, runs of T
-// consecutive parents, the 8 parity classes of a run adjacent (the plan's order).
-__global__ void noalloc_tiles_kernel(int4 *tiles, int depth, int T, int n_tiles) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n_tiles) return;
-  int rest = q;
-  for (int level = depth; level >= 2; --level) {
-    const int parents = 1 << (3 * (level - 1));
-    const int per_class = (parents + T - 1) / T;
-    if (rest < 8 * per_class) {
-      const int cls = rest & 7;
-      const int p0 = (rest >> 3) * T;
-      tiles[q] = make_int4(level, cls, p0, min(T, parents - p0));
-      return;
-    }
-    rest -= 8 * per_class;
-  }
-}
-
 } // namespace
 
 extern "C" int cdfmm_b200_evaluate_noalloc(cdfmm_b200_plan *plan, const cdfmm_b200_eval_args *a) {
@@ -123,22 +103,15 @@ extern "C" int cdfmm_b200_evaluate_noalloc(cdfmm_b200_plan *plan, const cdfmm_b2
   const int n = plan->n;
   const bool use_tc = plan->depth >= 2 && plan->tc_supported && K <= 128 &&
                       (plan->m2l_mode == CDFMM_B200_M2L_BF16X3 || plan->m2l_mode == CDFMM_B200_M2L_AUTO);
-  const int Kp = round_up(K, 8);
-  const int node_base = level_offset(2);
-  const int boxes = plan->n_nodes - node_base;
-  const int T = plan->tc_m_tiles * (128 / Kp);
-  int n_tiles = 0;
-  if (use_tc)
-    for (int level = plan->depth; level >= 2; --level) n_tiles += 8 * (((1 << (3 * (level - 1))) + T - 1) / T);
+  const int boxes = plan->n_nodes - level_offset(2);
   // Carve the scratch regions (each 256-byte aligned).
   const size_t mom_bytes = align256(sizeof(float4) * static_cast<size_t>(plan->ns) * moment_row(K));
   const size_t exp_bytes = align256(sizeof(float) * static_cast<size_t>(plan->n_nodes) * n * K);
   const size_t near_bytes = align256(sizeof(float4) * static_cast<size_t>(plan->nt) * K);
-  const size_t pack_bytes = use_tc ? align256(static_cast<size_t>(boxes + 1) * Kp * plan->tc_Kpad * 2) : 0;
-  const size_t tile_bytes = align256(sizeof(int4) * static_cast<size_t>(n_tiles));
+  const size_t pack_bytes = use_tc ? align256(m2l_operand_bytes(plan->depth, K, plan->tc_columns[0].chunks)) : 0;
   const size_t fold_bytes =
       (!use_tc && plan->depth >= 2) ? align256(sizeof(float) * static_cast<size_t>(boxes) * plan->tc_n_in * K) : 0;
-  const size_t need = mom_bytes + 2 * exp_bytes + near_bytes + 2 * pack_bytes + tile_bytes + fold_bytes;
+  const size_t need = mom_bytes + 2 * exp_bytes + near_bytes + pack_bytes + fold_bytes;
   if (need > kNoAllocScratchBytes)
     return noalloc_fail(plan, CDFMM_B200_ERR_INVALID_ARGUMENT,
                         "evaluate_noalloc needs " + std::to_string(need) + " bytes of scratch for this plan and n_states; "
@@ -161,9 +134,7 @@ extern "C" int cdfmm_b200_evaluate_noalloc(cdfmm_b200_plan *plan, const cdfmm_b2
   float *M = reinterpret_cast<float *>(take(exp_bytes));
   float *L = reinterpret_cast<float *>(take(exp_bytes));
   float4 *near = reinterpret_cast<float4 *>(take(near_bytes));
-  void *a_hi = take(pack_bytes);
-  void *a_lo = take(pack_bytes);
-  int4 *dtiles = reinterpret_cast<int4 *>(take(tile_bytes));
+  void *operand = take(pack_bytes);
   float *Mf = reinterpret_cast<float *>(take(fold_bytes));
 
   cudaStream_t s = static_cast<cudaStream_t>(a->stream);
@@ -172,7 +143,6 @@ extern "C" int cdfmm_b200_evaluate_noalloc(cdfmm_b200_plan *plan, const cdfmm_b2
   // as zero; the array still holds the previous call's values.
   e = cudaMemsetAsync(L, 0, exp_bytes, s);
   if (e != cudaSuccess) return noalloc_fail(plan, CDFMM_B200_ERR_RUNTIME, std::string("scratch: ") + cudaGetErrorString(e));
-  if (n_tiles > 0) noalloc_tiles_kernel<<<(n_tiles + 127) / 128, 128, 0, s>>>(dtiles, plan->depth, T, n_tiles);
 
   launch_gather_moments(a->moments, a->moments_dtype, plan->src_inv, plan->ns, K, plan->scale, mom, s,
                         moments_paired(K));
@@ -187,41 +157,32 @@ extern "C" int cdfmm_b200_evaluate_noalloc(cdfmm_b200_plan *plan, const cdfmm_b2
   launch_p2m(plan->src_rel, mom, plan->src_off, plan->basis, M, n, plan->p, K, plan->depth, plan->p2m_chunk, s,
              plan->cuboid_p2m ? plan->src_size : nullptr, plan->size_step);
   for (int level = plan->depth - 1; level >= 0; --level)
-    launch_m2m(M, plan->m2m_off, plan->m2m_pair, plan->m2m_coef, n, K, level, static_cast<int>(plan->ops.m2m_pair_g.size()), s);
+    launch_m2m(M, plan->m2m_coef, n, plan->p, K, level, s);
+  ReducedLocals red;
   if (use_tc) {
-    launch_m2l_pack(M, plan->scale_m, plan->tc_fold_off, plan->tc_fold, plan->tc_n_in, a_hi, a_lo, n, K, Kp,
-                    plan->tc_Kpad, plan->depth, node_base, boxes, s);
-    TcArgs ta{};
-    ta.a_hi = static_cast<const uint8_t *>(a_hi);
-    ta.a_lo = static_cast<const uint8_t *>(a_lo);
-    ta.b_tiles = static_cast<const uint8_t *>(plan->tc_b);
-    set_m2l_reduction(ta, plan);
-    ta.tiles = dtiles;
-    ta.scale_l = plan->scale_l;
-    ta.L = L;
-    ta.error_flag = plan->error_flag;
-    ta.n = n;
-    ta.K = K;
-    ta.Kp = Kp;
-    ta.Kpad = plan->tc_Kpad;
-    ta.Npad = plan->tc_Npad;
-    ta.node_base = node_base;
-    ta.zero_node = boxes;
-    ta.stages = plan->tc_stages;
-    ta.m_tiles = plan->tc_m_tiles;
-    ta.acc_stride = plan->tc_acc_stride;
-    ta.fuse_n = plan->tc_fuse;
-    ta.tmem_cols = plan->tc_tmem_cols;
-    ta.box_bytes = static_cast<uint32_t>(Kp) * static_cast<uint32_t>(plan->tc_Kpad) * 2u;
-    ta.wait_limit = plan->tc_wait_limit;
-    launch_m2l_tc(ta, n_tiles, s);
+    // The reduced locals of the M2L's splits take the scratch left over; one
+    // split needs none of it: once packed, the multipoles' region holds it.
+    const size_t split_bytes = sizeof(float) * cdfmm_b200_m2l_split_floats(plan, K);
+    const size_t left = kNoAllocScratchBytes - need;
+    const int room = static_cast<int>(std::min<size_t>(left / split_bytes, kM2lMaxSplits));
+    float *R = room >= 1 ? reinterpret_cast<float *>(cursor) : M;
+    M2lTcArgs ta;
+    try {
+      ta = cdfmm_b200_m2l_args(plan, K, operand, R, std::max(room, 1));
+    } catch (const std::exception &ex) {
+      return noalloc_fail(plan, CDFMM_B200_ERR_RUNTIME, ex.what());
+    }
+    launch_m2l_pack(M, plan->tc_fold_off, plan->tc_fold, plan->tc_n_fold, plan->tc_n_in, operand, n, K, ta.chunks,
+                    plan->depth, s);
+    launch_m2l_tc(ta, s);
+    red = reduced_locals(ta);
   } else if (plan->depth >= 2) {
     launch_m2l_simt(M, Mf, L, plan->m2l_T, plan->scale_m, plan->scale_l, plan->m2l_tiles, plan->n_tiles, n,
                     plan->m2l_ld_red, K, plan->depth, plan->tc_fold_off, plan->tc_fold, plan->tc_expand,
                     plan->tc_n_in, plan->tc_n_out, plan->tc_n_derived, s);
   }
-  for (int level = 3; level <= plan->depth; ++level)
-    launch_l2l(L, plan->l2l_off, plan->l2l_pair, plan->l2l_coef, n, K, level, static_cast<int>(plan->ops.l2l_pair_g.size()), s);
+  for (int level = use_tc ? 2 : 3; level <= plan->depth; ++level)
+    launch_l2l(L, plan->l2l_coef, n, plan->p, K, level, s, use_tc ? &red : nullptr);
   cudaStreamWaitEvent(s, plan->ev_join, 0);
   launch_l2p(L, plan->tgt_rel, plan->tgt_off, plan->tgt_perm, plan->tgt_inv, near, plan->basis, n, plan->p, K, plan->nt, plan->depth, a->output,
              a->layout, plan->phi_scale, a->field, a->potential, s);

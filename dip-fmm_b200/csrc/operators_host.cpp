@@ -107,27 +107,6 @@ HostOperators build_host_operators(int p, int depth, int m2l_ld_multiple) {
   ops.az = B.az;
   const int n = ops.n;
 
-  // Pair lists.  M2M: out alpha <- sum_{g <= alpha} c_g * in(alpha - g).
-  // L2L: out beta <- sum_{|beta + g| <= p} c_g * in(beta + g).
-  ops.m2m_off.assign(static_cast<std::size_t>(n) + 1, 0);
-  ops.l2l_off.assign(static_cast<std::size_t>(n) + 1, 0);
-  for (int a = 0; a < n; ++a) {
-    for (int g = 0; g < n; ++g) {
-      if (B.ax[g] <= B.ax[a] && B.ay[g] <= B.ay[a] && B.az[g] <= B.az[a]) {
-        ops.m2m_pair_g.push_back(g);
-        ops.m2m_pair_in.push_back(
-            BasisTable::rank(B.ax[a] - B.ax[g], B.ay[a] - B.ay[g], B.az[a] - B.az[g]));
-      }
-      const int sx = B.ax[a] + B.ax[g], sy = B.ay[a] + B.ay[g], sz = B.az[a] + B.az[g];
-      if (sx + sy + sz <= p) {
-        ops.l2l_pair_g.push_back(g);
-        ops.l2l_pair_in.push_back(BasisTable::rank(sx, sy, sz));
-      }
-    }
-    ops.m2m_off[a + 1] = static_cast<int>(ops.m2m_pair_g.size());
-    ops.l2l_off[a + 1] = static_cast<int>(ops.l2l_pair_g.size());
-  }
-
   // Shift coefficients per (level, child class) in normalised units: the
   // child half width at level l is 2^-(l+1) (root width 1); child offset from
   // its parent is +-half width per axis by the class bits (x=1, y=2, z=4).

@@ -95,13 +95,6 @@ template <typename T> T *grow_bytes(T *&buf, size_t &have, size_t need, const ch
   return buf;
 }
 
-// TMEM columns for m_tiles accumulators acc_stride apart (a power of two >= 32).
-uint32_t tmem_columns(int m_tiles, int acc_stride) {
-  uint32_t cols = 32;
-  while (cols < static_cast<uint32_t>(m_tiles * acc_stride)) cols <<= 1;
-  return cols;
-}
-
 // Grows a device buffer to at least `need` elements (contents not kept).
 template <typename T> T *grow(T *&buf, size_t &have, size_t need, const char *what) {
   if (have < need) {
@@ -117,10 +110,10 @@ template <typename T> T *grow(T *&buf, size_t &have, size_t need, const char *wh
 void free_plan(cdfmm_b200_plan *p) {
   if (p == nullptr) return;
   void *ptrs[] = {p->src_rel, p->tgt_rel, p->src_off, p->tgt_off, p->src_perm, p->tgt_perm, p->src_inv, p->tgt_inv,
-                  p->self_idx, p->leaf_self, p->p2p_work, p->m2m_off, p->m2m_pair, p->l2l_off, p->l2l_pair, p->m2m_coef,
+                  p->self_idx, p->leaf_self, p->p2p_work, p->m2m_coef,
                   p->l2l_coef, p->m2l_T, p->basis, p->mom, p->M, p->L, p->near, p->stage_in,
-                  p->stage_out, p->scale_m, p->scale_l, p->m2l_tiles, p->tc_a_hi, p->tc_a_lo,
-                  p->tc_b, p->m2l_fold_buf, p->tc_fold_off, p->tc_fold, p->tc_expand, p->tc_tiles, p->error_flag, p->wbuf, p->gpart, p->stage_grad, p->p2p_next_unit,
+                  p->stage_out, p->scale_m, p->scale_l, p->m2l_tiles, p->tc_a,
+                  p->tc_R, p->m2l_fold_buf, p->tc_fold_off, p->tc_fold, p->tc_expand, p->error_flag, p->wbuf, p->gpart, p->stage_grad, p->p2p_next_unit,
                   p->close_targets, p->close_r_fp32, p->close_r_exact, p->src_pos64, p->tgt_pos64,
                   p->src_size, p->src_size64, p->cuboid_T, p->cuboid_base, p->ntc_blk_off, p->ntc_blk_src,
                   p->ntc_blk_pos, p->ntc_work, p->ntc_b, p->ngt_blk_off, p->ngt_blk_src, p->ngt_blk_pos,
@@ -183,6 +176,42 @@ std::string timeout_message(int code, int calls, bool own) {
 }
 
 } // namespace
+
+size_t cdfmm_b200_m2l_split_floats(const cdfmm_b200_plan *plan, int K) {
+  return static_cast<size_t>(plan->n_nodes - level_offset(2)) * plan->tc_n_out * K;
+}
+
+int cdfmm_b200_m2l_splits(const cdfmm_b200_plan *plan, int K) {
+  // (the fused form's column groups may split a tile differently)
+  int most = 1;
+  for (const M2lColumns &c : plan->tc_columns)
+    most = std::max(most, m2l_grid(plan->depth, K, c, plan->tc_n_out, plan->sm_count, kM2lMaxSplits).splits);
+  return most;
+}
+
+M2lTcArgs cdfmm_b200_m2l_args(const cdfmm_b200_plan *plan, int K, void *a, float *R, int max_splits) {
+  const cdfmm_b200_plan::TcShape &shape = plan->tc_candidates[static_cast<size_t>(std::max(plan->tc_pinned, 0))];
+  const M2lColumns &c = plan->tc_columns[shape.fuse];
+  M2lTcArgs t{};
+  t.b = static_cast<const uint8_t *>(plan->tc_operator[shape.fuse]->b);
+  t.R = R;
+  t.split_stride = static_cast<long long>(cdfmm_b200_m2l_split_floats(plan, K));
+  t.error_flag = plan->error_flag;
+  t.depth = plan->depth;
+  t.K = K;
+  t.n_out = plan->tc_n_out;
+  t.groups = c.groups;
+  t.cols = c.cols;
+  t.chunks = c.chunks;
+  t.stages = shape.stages;
+  t.fused = shape.fuse;
+  t.tmem_cols = 32;
+  while (t.tmem_cols < static_cast<uint32_t>((shape.fuse ? 2 : 1) * c.cols)) t.tmem_cols <<= 1;
+  t.wait_limit = plan->tc_wait_limit;
+  if (!m2l_set_operand(t, m2l_grid(plan->depth, K, c, plan->tc_n_out, plan->sm_count, max_splits), a))
+    throw std::runtime_error("the M2L operand's tensor map could not be encoded");
+  return t;
+}
 
 cudaError_t cdfmm_b200_collect_status(cdfmm_b200_plan *plan, cudaStream_t s, unsigned long long call) {
   collect_status_kernel<<<1, 1, 0, s>>>(plan->error_flag, plan->status_dev, call);
@@ -298,20 +327,6 @@ int cdfmm_b200_device_info(int32_t device, char *name, size_t name_len, int32_t 
   if (cc_major) *cc_major = prop.major;
   if (cc_minor) *cc_minor = prop.minor;
   return CDFMM_B200_OK;
-}
-
-static size_t corun_m2l_smem_budget(const cdfmm_b200_plan *plan, int K);
-
-// BF16 hi/lo B tiles of the tensor-core M2L per (order, Npad, Kpad), packed
-// once per process and shared by the plans of that order.
-static std::shared_ptr<const std::vector<uint16_t>> packed_b_tiles(int p, const HostOperators &ops,
-                                                                    const M2lTraceless &red, int Npad, int Kpad) {
-  static std::mutex mutex;
-  static std::map<std::tuple<int, int, int>, std::shared_ptr<const std::vector<uint16_t>>> cache;
-  std::lock_guard<std::mutex> lock(mutex);
-  auto &slot = cache[std::make_tuple(p, Npad, Kpad)];
-  if (!slot) slot = std::make_shared<const std::vector<uint16_t>>(pack_m2l_b_tiles(*ops.m2l_T64, ops.n, red, Npad, Kpad));
-  return slot;
 }
 
 // A new plan's sizes, streams and events (root cube, geometry, operators
@@ -453,21 +468,10 @@ static void finish_plan(cdfmm_b200_plan *plan, int m2l_mode) {
     basis[4 * a + 2] = static_cast<int8_t>(ops.az[a]);
     basis[4 * a + 3] = static_cast<int8_t>(ops.ax[a] + ops.ay[a] + ops.az[a]);
   }
-  std::vector<int> m2m_pair(ops.m2m_pair_g.size()), l2l_pair(ops.l2l_pair_g.size());
-  for (size_t e = 0; e < m2m_pair.size(); ++e) m2m_pair[e] = ops.m2m_pair_g[e] | (ops.m2m_pair_in[e] << 16);
-  for (size_t e = 0; e < l2l_pair.size(); ++e) l2l_pair[e] = ops.l2l_pair_g[e] | (ops.l2l_pair_in[e] << 16);
   plan->basis = dalloc<int8_t>(basis.size(), bytes);
-  plan->m2m_off = dalloc<int>(ops.m2m_off.size(), bytes);
-  plan->l2l_off = dalloc<int>(ops.l2l_off.size(), bytes);
-  plan->m2m_pair = dalloc<int>(m2m_pair.size(), bytes);
-  plan->l2l_pair = dalloc<int>(l2l_pair.size(), bytes);
   plan->m2m_coef = dalloc<float>(ops.m2m_coef.size(), bytes);
   plan->l2l_coef = dalloc<float>(ops.l2l_coef.size(), bytes);
   upload(plan->basis, basis.data(), basis.size(), h2d);
-  upload(plan->m2m_off, ops.m2m_off.data(), ops.m2m_off.size(), h2d);
-  upload(plan->l2l_off, ops.l2l_off.data(), ops.l2l_off.size(), h2d);
-  upload(plan->m2m_pair, m2m_pair.data(), m2m_pair.size(), h2d);
-  upload(plan->l2l_pair, l2l_pair.data(), l2l_pair.size(), h2d);
   upload(plan->m2m_coef, ops.m2m_coef.data(), ops.m2m_coef.size(), h2d);
   upload(plan->l2l_coef, ops.l2l_coef.data(), ops.l2l_coef.size(), h2d);
 
@@ -501,6 +505,7 @@ static void finish_plan(cdfmm_b200_plan *plan, int m2l_mode) {
     plan->tc_n_in = static_cast<int>(red.in_set.size());
     plan->tc_n_out = static_cast<int>(red.out_set.size());
     plan->tc_n_derived = red.n_derived;
+    plan->tc_n_fold = static_cast<int>(red.fold.size());
     plan->tc_fold_off = dalloc<int>(red.fold_off.size(), bytes);
     upload(plan->tc_fold_off, red.fold_off.data(), red.fold_off.size(), h2d);
     plan->tc_fold = dalloc<int>(std::max<size_t>(red.fold.size(), 1), bytes);
@@ -595,6 +600,7 @@ static void finish_plan(cdfmm_b200_plan *plan, int m2l_mode) {
 
   const size_t smem = device_smem_optin(plan->device);
   configure_far_kernels(smem);
+  configure_shift_kernels(plan->p, smem);
   configure_m2l_simt(smem);
   configure_p2p(smem);
   plan->p2m_chunk = 64;
@@ -612,78 +618,46 @@ static void finish_plan(cdfmm_b200_plan *plan, int m2l_mode) {
   plan->tc_wait_limit = kTcWaitLimit;
 
   lap(plan->stats.setup_ms_buffers);
-  // Tensor-core M2L: sm_100 devices and at least two pipeline stages in
-  // shared memory (the traceless operator's N = 16 ceil((p+1)^2 / 16) <= 128
-  // accumulator columns for every order up to 10).  AUTO keeps order 10 on
-  // the FP32 SIMT M2L, whose products are exact FP32.
+  // Tensor-core M2L: sm_100 devices.  AUTO keeps order 10 on the FP32 SIMT
+  // M2L, whose products are exact FP32; AUTO and BF16X3 run any number of
+  // states up to 128 on the tensor cores, FP32 keeps the SIMT M2L (the plain
+  // per-state path).
   {
     int major = 0;
     cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, plan->device);
-    // traceless reduction: (p+1)^2 - 1 folded moments in, (p+1)^2 locals out
-    const M2lTraceless red = m2l_traceless(plan->p);
-    const int Kpad = std::max(16, round_up(static_cast<int>(red.in_set.size()), 16));
-    const int Npad = round_up(static_cast<int>(red.out_set.size()), 16);
-    // Pipeline shapes: 1, 2 or 4 128-row accumulators per CTA sharing each
-    // B tile, with as many stages as fit one CTA per SM, or half / a third
-    // of that for two / three CTAs per SM; each with the three products as
-    // three MMAs of N = Npad, or (when 2 Npad <= 256) A_hi x [B_hi | B_lo]
-    // fused into one MMA of N = 2 Npad plus A_lo x B_hi (two larger MMAs
-    // instead of three: fewer instructions for the one issuing thread;
-    // twice the TMEM columns).  Default: two accumulators, two CTAs per SM,
-    // three MMAs; the autotuner times the candidates on first use for
-    // each K.
-    auto acc_stride_of = [&](int fuse) { return round_up(fuse ? 2 * Npad : Npad, 32); };
-    auto max_stages = [&](int mt, size_t budget) {
-      int st = 0;
-      while (st < 8 && m2l_tc_smem_bytes(Npad, mt, st + 1, n) <= budget) ++st;
-      return st;
-    };
-    const size_t one_cta = std::min<size_t>(smem, 224 * 1024), two_cta = 112 * 1024, three_cta = 74 * 1024;
-    // one CTA beside two co-resident near-field CTAs (schedule CORUN)
-    const size_t corun_cta = corun_m2l_smem_budget(plan, std::min(plan->max_states, 64));
+    // Pipeline shapes: the stages that fit one CTA per SM, and half of that
+    // for two; each with the three products summed in one accumulator or
+    // (fused) the hi * lo product in columns of its own.  The default, first,
+    // is unfused: two CTAs per SM where two accumulators fit the SM's tensor
+    // memory (orders <= 4: one CTA's epilogue overlaps the other's MMAs), else
+    // the deepest pipeline of one.
     plan->tc_candidates.clear();
     for (int fuse : {0, 1}) {
-      if (fuse && 2 * Npad > 256) continue; // MMA N <= 256
-      const int acc = acc_stride_of(fuse);
-      for (int mt : {2, 1, 4}) {
-        if (mt * acc > 512) continue;
-        const int s1 = max_stages(mt, one_cta);
-        const int s2 = max_stages(mt, two_cta);
-        const int s3 = max_stages(mt, three_cta);
-        const int sc = max_stages(mt, corun_cta);
-        if (s2 >= 2 && s2 < s1 && tmem_columns(mt, acc) <= 256) plan->tc_candidates.push_back({mt, s2, fuse});
-        if (s1 >= 2) plan->tc_candidates.push_back({mt, s1, fuse});
-        if (s3 >= 2 && s3 < s2 && 3 * tmem_columns(mt, acc) <= 512) plan->tc_candidates.push_back({mt, s3, fuse});
-        if (sc >= 2 && sc != s1 && sc != s2 && sc != s3) plan->tc_candidates.push_back({mt, sc, fuse});
-      }
+      const M2lColumns c = m2l_columns(plan->p, fuse != 0);
+      plan->tc_columns[fuse] = c;
+      auto max_stages = [&](size_t budget) {
+        int st = 0;
+        while (st < kM2lMaxStages && m2l_tc_smem_bytes(c.cols, st + 1) <= budget) ++st;
+        return st;
+      };
+      const int one = max_stages(std::min<size_t>(smem, 224 * 1024)), two = max_stages(112 * 1024);
+      const bool pair = (fuse ? 2 : 1) * c.cols <= 256 && two >= 3;
+      if (pair) plan->tc_candidates.push_back({1, two, fuse});
+      if (one >= 2 && (!pair || one != two)) plan->tc_candidates.push_back({1, one, fuse});
+      if (!pair && two >= 2 && two != one) plan->tc_candidates.push_back({1, two, fuse});
     }
-    const int m_tiles = plan->tc_candidates.empty() ? 1 : plan->tc_candidates.front().m_tiles;
-    const int stages = plan->tc_candidates.empty() ? 0 : plan->tc_candidates.front().stages;
-    const int fuse0 = plan->tc_candidates.empty() ? 0 : plan->tc_candidates.front().fuse;
-    const int acc_stride = acc_stride_of(fuse0);
-    // AUTO and BF16X3 run the M2L on the tensor cores for any K (fewer
-    // than 8 states fill 8-row groups of the MMA tile with zero rows: the
-    // tensor cores still beat the FP32 SIMT M2L several times over);
-    // FP32 keeps the SIMT M2L (the plain per-state path).
     const bool wanted = m2l_mode == CDFMM_B200_M2L_BF16X3 || (m2l_mode == CDFMM_B200_M2L_AUTO && plan->p <= 9);
-    plan->tc_supported = major == 10 && plan->depth >= 2 && Npad <= 256 && stages >= 2 && wanted &&
+    plan->tc_supported = major == 10 && plan->depth >= 2 && !plan->tc_candidates.empty() && wanted &&
                          configure_m2l_tc(smem);
     if (plan->tc_supported) {
-      plan->tc_Kpad = Kpad;
-      plan->tc_Npad = Npad;
-      plan->tc_stages = stages;
-      plan->tc_m_tiles = m_tiles;
-      plan->tc_acc_stride = acc_stride;
-      plan->tc_fuse = fuse0;
-      plan->tc_tmem_cols = tmem_columns(m_tiles, acc_stride);
-      plan->tc_Kp_max = round_up(std::min(plan->max_states, 128), 8);
-      const size_t boxes = static_cast<size_t>(plan->n_nodes - level_offset(2)) + 1;
-      const size_t box_elems = static_cast<size_t>(plan->tc_Kp_max) * Kpad;
-      plan->tc_a_hi = dalloc<uint16_t>(boxes * box_elems, bytes);
-      plan->tc_a_lo = dalloc<uint16_t>(boxes * box_elems, bytes);
-      const std::shared_ptr<const std::vector<uint16_t>> bt = packed_b_tiles(plan->p, ops, red, Npad, Kpad);
-      plan->tc_b = dalloc<uint16_t>(bt->size(), bytes);
-      upload(static_cast<uint16_t *>(plan->tc_b), bt->data(), bt->size(), h2d);
+      plan->tc_operator[0] = m2l_operator(plan->device, plan->p, plan->tc_columns[0], *ops.m2l_T64);
+      const int k_max = std::min(plan->max_states, 128);
+      size_t r_floats = 0;
+      for (int k = 1; k <= k_max; ++k)
+        r_floats = std::max(r_floats, cdfmm_b200_m2l_split_floats(plan, k) *
+                                          static_cast<size_t>(cdfmm_b200_m2l_splits(plan, k)));
+      plan->tc_a = dalloc<uint8_t>(m2l_operand_bytes(plan->depth, k_max, plan->tc_columns[0].chunks), bytes);
+      plan->tc_R = dalloc<float>(r_floats, bytes);
     } else if (m2l_mode == CDFMM_B200_M2L_BF16X3) {
       throw AbiError(CDFMM_B200_ERR_RUNTIME,
                      "split-BF16 tensor-core M2L needs an sm_100 device and depth >= 2");
@@ -1044,105 +1018,6 @@ int cdfmm_b200_set_self_indices(cdfmm_b200_plan *plan, const int32_t *sorted_sel
   }
 }
 
-// Tensor-core M2L work tiles: per level (deepest first), runs of
-// T = m_tiles * (128 / Kp) consecutive parents in Morton order, the 8 parity
-// classes of a run adjacent so that CTAs running together read the same
-// source boxes (the run's parents' neighbours' children) from L2.
-static std::vector<int4> build_tc_tiles(int depth, int T) {
-  std::vector<int4> tiles;
-  for (int level = depth; level >= 2; --level) {
-    const int parents = 1 << (3 * (level - 1));
-    for (int p0 = 0; p0 < parents; p0 += T)
-      for (int cls = 0; cls < 8; ++cls) tiles.push_back(make_int4(level, cls, p0, std::min(T, parents - p0)));
-  }
-  return tiles;
-}
-
-static void upload_tc_tiles(cdfmm_b200_plan *plan, int Kp) {
-  const std::vector<int4> tiles = build_tc_tiles(plan->depth, plan->tc_m_tiles * (128 / Kp));
-  grow(plan->tc_tiles, plan->tc_tiles_capacity, tiles.size(), "cudaMalloc tiles");
-  copy_to_device(plan->tc_tiles, tiles.data(), tiles.size() * sizeof(int4), "tiles");
-  plan->tc_tiles_Kp = Kp;
-  plan->tc_n_tiles = static_cast<int>(tiles.size());
-}
-
-// Autotuner of the tensor-core M2L pipeline shape (accumulators per CTA,
-// stages, fused hi/lo B operand): times every candidate on this call's
-// packed operands (device events, second of two launches) and keeps the
-// fastest.  Candidates trade B reuse (more accumulators per CTA) against
-// pipeline depth, CTAs per SM and MMA size.  Shapes with the same fusion
-// give bit-identical results (the per-row MMA sequence is the same); the
-// fused form sums the hi*lo product in its own accumulator, a difference at
-// FP32 rounding level.
-static void tune_m2l_tc(cdfmm_b200_plan *plan, int K, cudaStream_t s, size_t smem_budget) {
-  const int Kp = round_up(K, 8);
-  const int node_base = level_offset(2);
-  TcArgs ta{};
-  ta.a_hi = static_cast<const uint8_t *>(plan->tc_a_hi);
-  ta.a_lo = static_cast<const uint8_t *>(plan->tc_a_lo);
-  ta.b_tiles = static_cast<const uint8_t *>(plan->tc_b); set_m2l_reduction(ta, plan);
-  ta.scale_l = plan->scale_l;
-  ta.L = plan->L;
-  ta.error_flag = plan->error_flag;
-  ta.n = plan->n;
-  ta.K = K;
-  ta.Kp = Kp;
-  ta.Kpad = plan->tc_Kpad;
-  ta.Npad = plan->tc_Npad;
-  ta.node_base = node_base;
-  ta.zero_node = plan->n_nodes - node_base;
-  ta.box_bytes = static_cast<uint32_t>(Kp) * static_cast<uint32_t>(plan->tc_Kpad) * 2u;
-  ta.wait_limit = plan->tc_wait_limit;
-  float best = 0.0F;
-  int best_i = -1;
-  // candidates within the budget (all of them if none fits)
-  auto launch_smem = [&](const cdfmm_b200_plan::TcShape &c) {
-    const int acc = round_up(c.fuse ? 2 * plan->tc_Npad : plan->tc_Npad, 32);
-    size_t b = m2l_tc_smem_bytes(plan->tc_Npad, c.m_tiles, c.stages, plan->n);
-    if (tmem_columns(c.m_tiles, acc) > 256) b = std::max<size_t>(b, 120 * 1024);
-    return b;
-  };
-  bool any_fits = false;
-  for (const cdfmm_b200_plan::TcShape &c : plan->tc_candidates) any_fits = any_fits || launch_smem(c) <= smem_budget;
-
-  for (size_t c = 0; c < plan->tc_candidates.size(); ++c) {
-    if (any_fits && launch_smem(plan->tc_candidates[c]) > smem_budget) continue;
-    const int mt = plan->tc_candidates[c].m_tiles;
-    const std::vector<int4> tiles = build_tc_tiles(plan->depth, mt * (128 / Kp));
-    grow(plan->tc_tiles, plan->tc_tiles_capacity, tiles.size(), "cudaMalloc tiles");
-    copy_to_device(plan->tc_tiles, tiles.data(), tiles.size() * sizeof(int4), "tiles");
-    ta.tiles = plan->tc_tiles;
-    ta.m_tiles = mt;
-    ta.stages = plan->tc_candidates[c].stages;
-    ta.fuse_n = plan->tc_candidates[c].fuse;
-    ta.acc_stride = round_up(ta.fuse_n ? 2 * plan->tc_Npad : plan->tc_Npad, 32);
-    ta.tmem_cols = tmem_columns(mt, ta.acc_stride);
-    // one warm-up launch, then the faster of two timed ones (single timings
-    // of neighbouring shapes differ by less than their run-to-run noise)
-    float ms = 0.0F;
-    for (int rep = 0; rep < 3; ++rep) {
-      check(cudaEventRecord(plan->ev_t[10], s), "event");
-      launch_m2l_tc(ta, static_cast<int>(tiles.size()), s);
-      check(cudaEventRecord(plan->ev_t[11], s), "event");
-      check(cudaEventSynchronize(plan->ev_t[11]), "autotune");
-      float t = 0.0F;
-      check(cudaEventElapsedTime(&t, plan->ev_t[10], plan->ev_t[11]), "event");
-      if (rep == 1 || (rep > 1 && t < ms)) ms = t;
-    }
-    if (best_i < 0 || ms < best) {
-      best = ms;
-      best_i = static_cast<int>(c);
-    }
-  }
-  const cdfmm_b200_plan::TcShape &best_shape = plan->tc_candidates[static_cast<size_t>(best_i)];
-  plan->tc_m_tiles = best_shape.m_tiles;
-  plan->tc_stages = best_shape.stages;
-  plan->tc_fuse = best_shape.fuse;
-  plan->tc_acc_stride = round_up(best_shape.fuse ? 2 * plan->tc_Npad : plan->tc_Npad, 32);
-  plan->tc_tmem_cols = tmem_columns(plan->tc_m_tiles, plan->tc_acc_stride);
-  plan->tc_tiles_Kp = 0; // rebuilt for the chosen shape by the caller
-}
-
 // Upward pass for K states whose sorted, scaled moments are in plan->mom:
 // P2M and M2M, leaving the multipoles in plan->M.  Returns the launch count.
 // With `ntc` (the tensor-core near field's moment blocks, packed for these
@@ -1159,8 +1034,7 @@ static int enqueue_upward(cdfmm_b200_plan *plan, int K, cudaStream_t s, bool tim
   ++launches;
   if (timing) check(cudaEventRecord(plan->ev_t[2], s), "event");
   for (int level = plan->depth - 1; level >= 0; --level) {
-    launch_m2m(plan->M, plan->m2m_off, plan->m2m_pair, plan->m2m_coef, n, K, level,
-               static_cast<int>(plan->ops.m2m_pair_g.size()), s);
+    launch_m2m(plan->M, plan->m2m_coef, n, plan->p, K, level, s);
     ++launches;
   }
   if (timing) check(cudaEventRecord(plan->ev_t[3], s), "event");
@@ -1258,39 +1132,22 @@ static int resolved_schedule(const cdfmm_b200_plan *plan, int K) {
   return plan->schedule == CDFMM_B200_SCHEDULE_CORUN ? CDFMM_B200_SCHEDULE_CORUN : CDFMM_B200_SCHEDULE_SEPARATE;
 }
 
-// Shared memory one tensor-core M2L CTA may use to sit beside two
-// co-resident near-field CTAs on one SM.
-static size_t corun_m2l_smem_budget(const cdfmm_b200_plan *plan, int K) {
-  int per_sm = 0, reserved = 0;
-  cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, plan->device);
-  cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, plan->device);
-  const size_t near = p2p_corun_cta_smem(K) + static_cast<size_t>(reserved);
-  const size_t used = 2 * near + static_cast<size_t>(reserved);
-  return static_cast<size_t>(per_sm) > used ? static_cast<size_t>(per_sm) - used : 0;
+// The plan's tensor-core M2L arguments for K states (kept for the last K and
+// shape: tensor maps and the tile choice depend on them alone).
+static const M2lTcArgs &m2l_args(cdfmm_b200_plan *plan, int K) {
+  if (!plan->tc_args) plan->tc_args = std::make_unique<M2lTcArgs>();
+  if (plan->tc_args->K != K)
+    *plan->tc_args = cdfmm_b200_m2l_args(plan, K, plan->tc_a, plan->tc_R, cdfmm_b200_m2l_splits(plan, K));
+  plan->tc_args->wait_limit = plan->tc_wait_limit;
+  return *plan->tc_args;
 }
 
-// Tensor-core M2L operands: packs the scaled multipoles into BF16 hi/lo boxes
-// and, on the first use for this K (or after a schedule change), chooses the
-// pipeline shape -- the fastest candidate whose shared memory fits beside
-// the co-resident near field when K states run CORUN -- and builds its work
-// tiles.  Every path of the plan (device or host arrays, backward) then
-// uses that shape.  Returns the launch count.
+// Tensor-core M2L operand: folds, scales and splits the multipoles of levels
+// 2..depth.  Returns the launch count.
 static int prepare_m2l(cdfmm_b200_plan *plan, int K, cudaStream_t s) {
   if (!m2l_on_tensor_cores(plan, K)) return 0;
-  const size_t smem_budget =
-      resolved_schedule(plan, K) == CDFMM_B200_SCHEDULE_CORUN ? corun_m2l_smem_budget(plan, K) : SIZE_MAX;
-  const int Kp = round_up(K, 8);
-  const int node_base = level_offset(2);
-  const int boxes = plan->n_nodes - node_base;
-  launch_m2l_pack(plan->M, plan->scale_m, plan->tc_fold_off, plan->tc_fold, plan->tc_n_in, plan->tc_a_hi, plan->tc_a_lo,
-                  plan->n, K, Kp, plan->tc_Kpad,
-                  plan->depth, node_base, boxes, s);
-  if (plan->tc_tiles_Kp != Kp || (!plan->tc_pinned && plan->tc_tuned_budget != smem_budget)) {
-    check(cudaStreamSynchronize(s), "sync");
-    if (plan->tc_candidates.size() > 1 && !plan->tc_pinned) tune_m2l_tc(plan, K, s, smem_budget);
-    plan->tc_tuned_budget = smem_budget;
-    upload_tc_tiles(plan, Kp);
-  }
+  launch_m2l_pack(plan->M, plan->tc_fold_off, plan->tc_fold, plan->tc_n_fold, plan->tc_n_in, plan->tc_a, plan->n, K,
+                  plan->tc_columns[0].chunks, plan->depth, s);
   return 1;
 }
 
@@ -1300,52 +1157,30 @@ static int prepare_m2l(cdfmm_b200_plan *plan, int K, cudaStream_t s) {
 static int enqueue_downward(cdfmm_b200_plan *plan, int K, cudaStream_t s, bool timing, bool prepared = false) {
   const int n = plan->n;
   int launches = 0;
-    const bool use_tc = m2l_on_tensor_cores(plan, K);
-    if (use_tc) {
-      if (!prepared) launches += prepare_m2l(plan, K, s);
-      const int Kp = round_up(K, 8);
-      const int node_base = level_offset(2);
-      const int boxes = plan->n_nodes - node_base;
-      TcArgs ta{};
-      ta.a_hi = static_cast<const uint8_t *>(plan->tc_a_hi);
-      ta.a_lo = static_cast<const uint8_t *>(plan->tc_a_lo);
-      ta.b_tiles = static_cast<const uint8_t *>(plan->tc_b); set_m2l_reduction(ta, plan);
-      ta.tiles = plan->tc_tiles;
-      ta.scale_l = plan->scale_l;
-      ta.L = plan->L;
-      ta.error_flag = plan->error_flag;
-      ta.n = n;
-      ta.K = K;
-      ta.Kp = Kp;
-      ta.Kpad = plan->tc_Kpad;
-      ta.Npad = plan->tc_Npad;
-      ta.node_base = node_base;
-      ta.zero_node = boxes;
-      ta.stages = plan->tc_stages;
-      ta.m_tiles = plan->tc_m_tiles;
-      ta.acc_stride = plan->tc_acc_stride;
-      ta.fuse_n = plan->tc_fuse;
-      ta.tmem_cols = plan->tc_tmem_cols;
-      ta.box_bytes = static_cast<uint32_t>(Kp) * static_cast<uint32_t>(plan->tc_Kpad) * 2u;
-      ta.wait_limit = plan->tc_wait_limit;
-      launch_m2l_tc(ta, plan->tc_n_tiles, s);
-      launches += 1;
-      plan->stats.m2l_tc_m_tiles = plan->tc_m_tiles;
-      plan->stats.m2l_tc_stages = plan->tc_stages;
-      plan->stats.m2l_tc_fused = plan->tc_fuse;
-    } else if (plan->depth >= 2) {
-      launch_m2l_simt(plan->M, plan->m2l_fold_buf, plan->L, plan->m2l_T, plan->scale_m, plan->scale_l,
-                      plan->m2l_tiles, plan->n_tiles, n, plan->m2l_ld_red, K, plan->depth, plan->tc_fold_off,
-                      plan->tc_fold, plan->tc_expand, plan->tc_n_in, plan->tc_n_out, plan->tc_n_derived, s);
-      ++launches;
-    }
-    plan->last_m2l_tc = use_tc;
-    if (timing) check(cudaEventRecord(plan->ev_t[4], s), "event");
-    for (int level = 3; level <= plan->depth; ++level) {
-      launch_l2l(plan->L, plan->l2l_off, plan->l2l_pair, plan->l2l_coef, n, K, level,
-                 static_cast<int>(plan->ops.l2l_pair_g.size()), s);
-      ++launches;
-    }
+  const bool use_tc = m2l_on_tensor_cores(plan, K);
+  ReducedLocals red;
+  if (use_tc) {
+    if (!prepared) launches += prepare_m2l(plan, K, s);
+    const M2lTcArgs &ta = m2l_args(plan, K);
+    launches += launch_m2l_tc(ta, s);
+    red = reduced_locals(ta);
+    const cdfmm_b200_plan::TcShape &shape =
+        plan->tc_candidates[static_cast<size_t>(std::max(plan->tc_pinned, 0))];
+    plan->stats.m2l_tc_m_tiles = shape.m_tiles;
+    plan->stats.m2l_tc_stages = shape.stages;
+    plan->stats.m2l_tc_fused = shape.fuse;
+  } else if (plan->depth >= 2) {
+    launch_m2l_simt(plan->M, plan->m2l_fold_buf, plan->L, plan->m2l_T, plan->scale_m, plan->scale_l,
+                    plan->m2l_tiles, plan->n_tiles, n, plan->m2l_ld_red, K, plan->depth, plan->tc_fold_off,
+                    plan->tc_fold, plan->tc_expand, plan->tc_n_in, plan->tc_n_out, plan->tc_n_derived, s);
+    ++launches;
+  }
+  plan->last_m2l_tc = use_tc;
+  if (timing) check(cudaEventRecord(plan->ev_t[4], s), "event");
+  for (int level = use_tc ? 2 : 3; level <= plan->depth; ++level) {
+    launch_l2l(plan->L, plan->l2l_coef, n, plan->p, K, level, s, use_tc ? &red : nullptr);
+    ++launches;
+  }
   return launches;
 }
 
@@ -1474,10 +1309,10 @@ void cdfmm_b200_stacked_upward(cdfmm_b200_plan *plan, const cdfmm_b200_eval_args
   check(cudaGetLastError(), "kernel launch");
 }
 
-void cdfmm_b200_stacked_downward(cdfmm_b200_plan *plan, const cdfmm_b200_eval_args *a, cudaStream_t s) {
-  for (int level = 3; level <= plan->depth; ++level)
-    launch_l2l(plan->L, plan->l2l_off, plan->l2l_pair, plan->l2l_coef, plan->n, 1, level,
-               static_cast<int>(plan->ops.l2l_pair_g.size()), s);
+void cdfmm_b200_stacked_downward(cdfmm_b200_plan *plan, const cdfmm_b200_eval_args *a, cudaStream_t s,
+                                 const ReducedLocals &red) {
+  for (int level = 2; level <= plan->depth; ++level)
+    launch_l2l(plan->L, plan->l2l_coef, plan->n, plan->p, 1, level, s, &red);
   check(cudaStreamWaitEvent(s, plan->ev_join, 0), "wait");
   launch_l2p(plan->L, plan->tgt_rel, plan->tgt_off, plan->tgt_perm, plan->tgt_inv, plan->near, plan->basis, plan->n,
              plan->p, 1, plan->nt, plan->depth, a->output, a->layout, plan->phi_scale, a->field, a->potential, s);
@@ -2039,23 +1874,29 @@ int cdfmm_b200_m2l_shapes(const cdfmm_b200_plan *plan, int32_t *out, int32_t cap
 int cdfmm_b200_set_m2l_shape(cdfmm_b200_plan *plan, int32_t m_tiles, int32_t stages, int32_t fused) {
   if (plan == nullptr) return fail(nullptr, CDFMM_B200_ERR_INVALID_ARGUMENT, "plan is NULL");
   if (m_tiles == 0) {
-    plan->tc_pinned = false;
-    plan->tc_tiles_Kp = 0; // re-tune on the next tensor-core evaluate
+    plan->tc_pinned = -1;
+    plan->tc_args.reset();
     return CDFMM_B200_OK;
   }
   if (!plan->tc_supported)
     return fail(plan, CDFMM_B200_ERR_INVALID_ARGUMENT, "this plan has no tensor-core M2L (m2l_mode, order or device)");
-  for (const cdfmm_b200_plan::TcShape &c : plan->tc_candidates) {
-    if (c.m_tiles == m_tiles && c.stages == stages && c.fuse == (fused != 0 ? 1 : 0)) {
-      plan->tc_m_tiles = c.m_tiles;
-      plan->tc_stages = c.stages;
-      plan->tc_fuse = c.fuse;
-      plan->tc_acc_stride = round_up(c.fuse ? 2 * plan->tc_Npad : plan->tc_Npad, 32);
-      plan->tc_tmem_cols = tmem_columns(plan->tc_m_tiles, plan->tc_acc_stride);
-      plan->tc_pinned = true;
-      plan->tc_tiles_Kp = 0; // work tiles rebuilt for this shape on the next evaluate
-      return CDFMM_B200_OK;
+  for (size_t i = 0; i < plan->tc_candidates.size(); ++i) {
+    const cdfmm_b200_plan::TcShape &c = plan->tc_candidates[i];
+    if (c.m_tiles != m_tiles || c.stages != stages || c.fuse != (fused != 0 ? 1 : 0)) continue;
+    try {
+      if (!plan->tc_operator[c.fuse]) {
+        check(cudaSetDevice(plan->device), "cudaSetDevice");
+        plan->tc_operator[c.fuse] =
+            m2l_operator(plan->device, plan->p, plan->tc_columns[c.fuse], *m2l_matrices(plan->p));
+      }
+    } catch (const std::bad_alloc &) {
+      return fail(plan, CDFMM_B200_ERR_OUT_OF_MEMORY, "allocation of the M2L operator tiles failed");
+    } catch (const std::exception &e) {
+      return fail(plan, CDFMM_B200_ERR_RUNTIME, e.what());
     }
+    plan->tc_pinned = static_cast<int>(i);
+    plan->tc_args.reset();
+    return CDFMM_B200_OK;
   }
   return fail(plan, CDFMM_B200_ERR_INVALID_ARGUMENT,
               "not a pipeline shape of this plan (cdfmm_b200_m2l_shapes lists them)");
@@ -2293,8 +2134,6 @@ const char *cdfmm_b200_last_error(const cdfmm_b200_plan *plan) {
 
 } // extern "C"
 
-std::vector<int4> cdfmm_b200::tc_work_tiles(int depth, int T) { return build_tc_tiles(depth, T); }
-uint32_t cdfmm_b200::tc_tmem_columns(int m_tiles, int acc_stride) { return tmem_columns(m_tiles, acc_stride); }
 
 cdfmm_b200::CloseGeometry cdfmm_b200_near_geometry(const cdfmm_b200_plan *plan) {
   using cdfmm_b200::CloseGeometry;

@@ -1,0 +1,424 @@
+// M2M and L2L: shifts of expansions between a parent and its 8 children.
+//
+// The shift of a Taylor expansion by h is a tensor product of three
+// one-dimensional shifts, because h^g / g! = prod over axes h_a^g_a / g_a!:
+//   L2L: L'[b] = sum_g h^g/g! L[b + g]   = shift_z(shift_y(shift_x(L)))
+//   M2M: M'[a] = sum_g h^g/g! M[a - g]
+// Along one axis the coefficients with the two other indices fixed form a
+// line of p + 1 - (their sum) values, and a 1-D shift of a line of m values
+// is m (m + 1) / 2 FMAs: 210 FMAs per axis at p = 6 where the full pair list
+// has 924 (495 against 3003 at p = 8).  The two children of one axis sit at
+// +-h, so their even and odd powers are shared: M2M shifts the sum and the
+// difference of the two lines, L2L forms both children from one even and one
+// odd sum.  Per parent and state that is 7 x 210 FMAs instead of 8 x 924.
+//
+// A CTA takes 32 columns, a column being one state of one parent: one parent
+// and up to 32 states where K >= 32, else as many whole parents as fit.  A
+// lane owns a column, so every shared-memory access of a warp is one row of
+// 32 consecutive floats and a line's values live in registers; a warp takes
+// whole lines.  The kernels are compiled per order with the lines unrolled:
+// every rank is then a constant, and a line is its loads, FMAs and stores
+// (computing the ranks per element took more instructions than the shift).
+// Bound: HBM (the children's expansions, read once by M2M and written once by
+// L2L) and shared-memory access.  Measured over a depth-5 tree (before: the
+// full pair list from shared memory, L2L reading and rewriting the locals):
+// p = 6, K = 64 M2M 0.98 -> 0.27 ms, L2L 0.69 -> 0.70 ms with the expansion;
+// p = 8, K = 64 M2M 4.5 -> 0.92 ms; p = 6, K = 1 M2M 159 -> 80 us, L2L 130 ->
+// 54 us.
+// Upstream math: src/far_field.cpp:303-331 (M2M), :533-581 (L2L).
+#include <cuda_runtime.h>
+
+#include <type_traits>
+
+#include "far_kernels.hpp"
+#include "kernels.cuh"
+
+namespace cdfmm_b200 {
+
+namespace {
+
+constexpr int kCols = 32;          // columns (parent, state) of a CTA
+constexpr int kPitch = kCols + 1;  // shared row pitch: conflict-free by column and by coefficient
+constexpr int kShiftWarps = 8;
+constexpr int kShiftThreads = 32 * kShiftWarps;
+
+// Rank of element i of the line (u, w) of an axis.
+template <int AXIS> __device__ __forceinline__ int line_rank(int u, int w, int i) {
+  return AXIS == 0 ? rank3(i, u, w) : AXIS == 1 ? rank3(u, i, w) : rank3(u, w, i);
+}
+
+// h^g / g! of one axis from a class row of the shift table.
+template <int AXIS, int P>
+__device__ __forceinline__ void axis_coefficients(const float *__restrict__ row, float (&c)[P + 1]) {
+#pragma unroll
+  for (int g = 0; g <= P; ++g) c[g] = __ldg(row + line_rank<AXIS>(0, 0, g));
+}
+
+// Calls f(u, w, m) with compile-time exponents and length m = P + 1 - u - w
+// for this warp's lines of one axis, in order of falling length.
+template <int P, int D = 0, int U = 0, int Q = 0, class F> __device__ __forceinline__ void for_lines(int warp, F f) {
+  if constexpr (D <= P) {
+    if (Q % kShiftWarps == warp)
+      f(std::integral_constant<int, U>{}, std::integral_constant<int, D - U>{}, std::integral_constant<int, P + 1 - D>{});
+    if constexpr (U < D)
+      for_lines<P, D, U + 1, Q + 1>(warp, f);
+    else
+      for_lines<P, D + 1, 0, Q + 1>(warp, f);
+  }
+}
+
+// The columns of one CTA: `np` parents from `parent0` with `kc` states from
+// `kb`; rows of a node are K states long.
+struct Columns {
+  long long parent0;
+  int np, kb, kc, pi, k; // this lane: parent pi of the CTA, state kb + k
+  bool valid;
+};
+
+__device__ __forceinline__ Columns columns(long long n_parents, int nP, int K) {
+  Columns c;
+  c.parent0 = static_cast<long long>(blockIdx.x) * nP;
+  c.np = static_cast<int>(min(static_cast<long long>(nP), n_parents - c.parent0));
+  c.kb = blockIdx.y * kCols;
+  c.kc = min(kCols, K - c.kb);
+  const int lane = threadIdx.x & 31;
+  c.pi = lane / c.kc;
+  c.k = lane - c.pi * c.kc;
+  c.valid = c.pi < c.np;
+  if (!c.valid) c.pi = 0;
+  return c;
+}
+
+// Copies `rows` coefficient rows of the CTA's columns between shared memory
+// and the nodes (first + pi * step): rows of states where a parent fills the
+// CTA, else the contiguous run of each node (K states of every row).
+template <class Op>
+__device__ __forceinline__ void for_node_rows(const Columns &c, int rows, int K, long long first, long long step, Op op) {
+  if (K > kCols) {
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < rows; r += blockDim.x >> 5)
+      if (lane < c.kc) op((first * rows + r) * K + c.kb + lane, r * kPitch + lane);
+  } else {
+    const int run = rows * K;
+    for (int e = threadIdx.x; e < c.np * run; e += blockDim.x) {
+      const int pi = e / run;
+      const int t = e - pi * run;
+      const int r = K == 1 ? t : t / K;
+      op((first + pi * step) * run + t, r * kPitch + pi * c.kc + (t - r * K));
+    }
+  }
+}
+
+// M2M for one parent level.  z-lines of the children come straight from
+// global memory (four children per thread), then y and x in shared memory.
+template <int P>
+__global__ void __launch_bounds__(kShiftThreads, P <= 6 ? 4 : P <= 8 ? 3 : 2)
+    m2m_kernel(float *__restrict__ M, const float *__restrict__ coef, int K, int parent_level, long long n_parents,
+               int nP) {
+  constexpr int n = (P + 1) * (P + 2) * (P + 3) / 6;
+  constexpr int plane = n * kPitch;
+  extern __shared__ float sh[]; // [4 (x, y child)][n][kPitch]
+  const Columns col = columns(n_parents, nP, K);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float *row = coef + 7 * n; // class 7: the + child of every axis
+  const long long child0 = level_offset_d(parent_level + 1) + (col.parent0 + col.pi) * 8;
+  const long long per = static_cast<long long>(n) * K;
+  float c[P + 1];
+  // out[i] = sum_{g even} c_g (plus + minus)[i - g] + sum_{g odd} c_g (plus - minus)[i - g]
+  auto combine = [&](auto M_, float *s, float *d, auto store) {
+    constexpr int m = decltype(M_)::value;
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      const float a = s[i], b = d[i];
+      s[i] = a + b;
+      d[i] = a - b;
+    }
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      float v = 0.0F;
+#pragma unroll
+      for (int g = 0; g <= i; ++g) v = fmaf(c[g], (g & 1) ? d[i - g] : s[i - g], v);
+      store(i, v);
+    }
+  };
+  axis_coefficients<2, P>(row, c);
+#pragma unroll 1
+  for (int x = 0; x < 2; ++x) {
+    const float *src = M + (child0 + x) * per + col.kb + col.k;
+    float *dst = sh + x * plane + lane;
+    for_lines<P>(warp, [&](auto U_, auto W_, auto M_) {
+      // one line of the four children (y = 0 / 1, z = - / +): all its loads
+      // are in flight together
+      constexpr int u = decltype(U_)::value, w = decltype(W_)::value, m = decltype(M_)::value;
+      float s[2][m], d[2][m];
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int i = 0; i < m; ++i) {
+          const float *at = src + line_rank<2>(u, w, i) * K + 2 * y * per;
+          s[y][i] = col.valid ? at[4 * per] : 0.0F;
+          d[y][i] = col.valid ? at[0] : 0.0F;
+        }
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+        combine(M_, s[y], d[y], [&](int i, float v) { dst[2 * y * plane + line_rank<2>(u, w, i) * kPitch] = v; });
+    });
+  }
+  __syncthreads();
+  axis_coefficients<1, P>(row, c);
+#pragma unroll 1
+  for (int x = 0; x < 2; ++x) {
+    float *at = sh + x * plane + lane;
+    for_lines<P>(warp, [&](auto U_, auto W_, auto M_) {
+      constexpr int u = decltype(U_)::value, w = decltype(W_)::value, m = decltype(M_)::value;
+      float s[m], d[m];
+#pragma unroll
+      for (int i = 0; i < m; ++i) {
+        s[i] = at[2 * plane + line_rank<1>(u, w, i) * kPitch];
+        d[i] = at[line_rank<1>(u, w, i) * kPitch];
+      }
+      combine(M_, s, d, [&](int i, float v) { at[line_rank<1>(u, w, i) * kPitch] = v; });
+    });
+  }
+  __syncthreads();
+  axis_coefficients<0, P>(row, c);
+  const bool direct = K > kCols;
+  float *out = M + (level_offset_d(parent_level) + col.parent0) * per + col.kb + col.k;
+  float *at = sh + lane;
+  for_lines<P>(warp, [&](auto U_, auto W_, auto M_) {
+    constexpr int u = decltype(U_)::value, w = decltype(W_)::value, m = decltype(M_)::value;
+    float s[m], d[m];
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      s[i] = at[plane + line_rank<0>(u, w, i) * kPitch];
+      d[i] = at[line_rank<0>(u, w, i) * kPitch];
+    }
+    combine(M_, s, d, [&](int i, float v) {
+      if (!direct)
+        at[line_rank<0>(u, w, i) * kPitch] = v;
+      else if (col.valid)
+        out[line_rank<0>(u, w, i) * K] = v;
+    });
+  });
+  if (direct) return;
+  __syncthreads();
+  for_node_rows(col, n, K, level_offset_d(parent_level) + col.parent0, 1,
+                [&](long long g, int s) { M[g] = sh[s]; });
+}
+
+// Position of reduced local (a, b, r) (r = z exponent, 0 or 1) among the
+// (p + 1)^2 of M2lTraceless::out_set: degree d starts at d^2 and holds, per
+// a, first z = 1 then z = 0.
+__device__ __forceinline__ int reduced_index(int a, int b, int r) {
+  const int d = a + b + r;
+  return d * d + 2 * a + (r == 0 && b > 0 ? 1 : 0);
+}
+
+// Local (u, w, I) from the reduced ones of one child (column of rows of
+// kPitch), by the trace relations L_b = -L_{b-2z+2x} - L_{b-2z+2y} applied
+// I / 2 times: (-1)^k sum_t C(k, t) L_(u + 2t, w + 2(k - t), I mod 2).
+template <int I> __device__ __forceinline__ float local_from_reduced(const float *red, int u, int w) {
+  constexpr int k = I / 2, r = I & 1;
+  float v = 0.0F;
+  int c = (k & 1) ? -1 : 1;
+#pragma unroll
+  for (int t = 0; t <= k; ++t) {
+    v = fmaf(static_cast<float>(c), red[reduced_index(u + 2 * t, w + 2 * (k - t), r) * kPitch], v);
+    c = c * (k - t) / (t + 1);
+  }
+  return v;
+}
+
+// Calls f(integral_constant 0), ..., f(integral_constant M - 1).
+template <int M, class F> __device__ __forceinline__ void unrolled(F f) {
+  if constexpr (M > 0) {
+    unrolled<M - 1>(f);
+    f(std::integral_constant<int, M - 1>{});
+  }
+}
+
+// L2L for one child level; blockIdx.z is the (x, y) child pair.  EXPAND: the
+// children's locals are written as the M2L's reduced locals (summed over its
+// splits, scaled by 2^(l (|b| + 1)), the rest from the trace relations) plus
+// the shifted parent; else the shifted parent is added to the locals there.
+template <int P, bool EXPAND>
+__global__ void __launch_bounds__(kShiftThreads, P <= 6 ? 4 : P <= 8 ? 3 : 2)
+    l2l_kernel(float *__restrict__ L, const float *__restrict__ coef, int K, int child_level, long long n_parents,
+               int nP, const ReducedLocals red) {
+  constexpr int n = (P + 1) * (P + 2) * (P + 3) / 6, n_out = (P + 1) * (P + 1);
+  extern __shared__ float sh[]; // two planes [n][kPitch], reduced locals of the two z children [2][n_out][kPitch]
+  const Columns col = columns(n_parents, nP, K);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int xy = blockIdx.z;
+  const float *row = coef + (4 + xy) * n; // class (x, y, +z)
+  const bool shifted = !EXPAND || child_level > 2; // locals of levels 0 and 1 are zero
+  float *sA = sh, *sB = sh + n * kPitch, *sR = sB + n * kPitch;
+  const long long child0 = level_offset_d(child_level) + col.parent0 * 8 + xy; // -z child; +z is 4 further
+  const long long per4 = 4LL * n * K;
+  if constexpr (EXPAND) {
+    const long long box0 = child0 - level_offset_d(2);
+    auto load = [&](int z, int pi, int j, int k, int c) {
+      cp_async4(sR + (z * n_out + j) * kPitch + c,
+                red.R + ((box0 + pi * 8 + 4 * z) * n_out + j) * red.ld + red.k0 + k);
+    };
+    if (K > kCols) {
+      for (int r = warp; r < 2 * n_out; r += kShiftWarps)
+        if (lane < col.kc) load(r >= n_out, 0, r >= n_out ? r - n_out : r, col.kb + lane, lane);
+    } else {
+      const int run = n_out * K;
+      for (int e = threadIdx.x; e < 2 * col.np * run; e += kShiftThreads) {
+        const int t = e / run, q = e - t * run;
+        const int j = K == 1 ? q : q / K;
+        load(t & 1, t >> 1, j, q - j * K, (t >> 1) * K + q - j * K);
+      }
+    }
+  }
+  float c[P + 1];
+  auto shift = [&](auto M_, const float *v, auto store) {
+    constexpr int m = decltype(M_)::value;
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      float x = 0.0F;
+#pragma unroll
+      for (int g = 0; i + g < m; ++g) x = fmaf(c[g], v[i + g], x);
+      store(i, x);
+    }
+  };
+  if (shifted) {
+    for_node_rows(col, n, K, level_offset_d(child_level - 1) + col.parent0, 1,
+                  [&](long long g, int s) { cp_async4(sA + s, L + g); });
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  if (shifted) {
+    axis_coefficients<0, P>(row, c);
+    __syncthreads();
+    for_lines<P>(warp, [&](auto U_, auto W_, auto M_) {
+      constexpr int u = decltype(U_)::value, w = decltype(W_)::value, m = decltype(M_)::value;
+      float v[m];
+#pragma unroll
+      for (int i = 0; i < m; ++i) v[i] = sA[line_rank<0>(u, w, i) * kPitch + lane];
+      shift(M_, v, [&](int i, float x) { sB[line_rank<0>(u, w, i) * kPitch + lane] = x; });
+    });
+    axis_coefficients<1, P>(row, c);
+    __syncthreads();
+    for_lines<P>(warp, [&](auto U_, auto W_, auto M_) {
+      constexpr int u = decltype(U_)::value, w = decltype(W_)::value, m = decltype(M_)::value;
+      float v[m];
+#pragma unroll
+      for (int i = 0; i < m; ++i) v[i] = sB[line_rank<1>(u, w, i) * kPitch + lane];
+      shift(M_, v, [&](int i, float x) { sA[line_rank<1>(u, w, i) * kPitch + lane] = x; });
+    });
+  }
+  axis_coefficients<2, P>(row, c);
+  __syncthreads();
+  const bool direct = K > kCols;
+  const bool store = direct && col.valid;
+  float *out = L + child0 * n * K + col.kb + col.k;
+  for_lines<P>(warp, [&](auto U_, auto W_, auto M_) {
+    constexpr int u = decltype(U_)::value, w = decltype(W_)::value, m = decltype(M_)::value;
+    float v[m], lo[m], hi[m]; // the line, and the two children's locals
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      if constexpr (!EXPAND) {
+        // every load ahead of the stores below, which may alias them
+        lo[i] = store ? out[line_rank<2>(u, w, i) * K] : 0.0F;
+        hi[i] = store ? out[line_rank<2>(u, w, i) * K + per4] : 0.0F;
+      }
+      v[i] = shifted ? sA[line_rank<2>(u, w, i) * kPitch + lane] : 0.0F;
+    }
+    if constexpr (EXPAND)
+      unrolled<m>([&](auto I_) {
+        constexpr int i = decltype(I_)::value;
+        const float scale = __int_as_float((127 + child_level * (u + w + i + 1)) << 23);
+        lo[i] = scale * local_from_reduced<i>(sR + lane, u, w);
+        hi[i] = scale * local_from_reduced<i>(sR + n_out * kPitch + lane, u, w);
+      });
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      float e = 0.0F, o = 0.0F;
+#pragma unroll
+      for (int g = 0; i + g < m; ++g) {
+        if (g & 1)
+          o = fmaf(c[g], v[i + g], o);
+        else
+          e = fmaf(c[g], v[i + g], e);
+      }
+      lo[i] += e - o;
+      hi[i] += e + o;
+    }
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      const int r = line_rank<2>(u, w, i);
+      if (!direct) {
+        sA[r * kPitch + lane] = lo[i];
+        sB[r * kPitch + lane] = hi[i];
+      } else if (store) {
+        out[r * K] = lo[i];
+        out[r * K + per4] = hi[i];
+      }
+    }
+  });
+  if (direct) return;
+  __syncthreads();
+  for_node_rows(col, n, K, child0, 8, [&](long long g, int s) {
+    L[g] = EXPAND ? sA[s] : L[g] + sA[s];
+    L[g + per4] = EXPAND ? sB[s] : L[g + per4] + sB[s];
+  });
+}
+
+// Whole parents per CTA.
+int parents_per_cta(int K) { return K >= kCols ? 1 : kCols / K; }
+
+// Calls f with the order as a compile-time constant.
+template <int P = 0, class F> void with_order(int p, F f) {
+  if constexpr (P <= 10) {
+    if (p == P)
+      f(std::integral_constant<int, P>{});
+    else
+      with_order<P + 1>(p, f);
+  }
+}
+
+} // namespace
+
+void launch_m2m(float *M, const float *coef, int n, int p, int K, int parent_level, cudaStream_t s) {
+  const long long parents = 1LL << (3 * parent_level);
+  const int nP = parents_per_cta(K);
+  const dim3 grid(static_cast<unsigned>((parents + nP - 1) / nP), static_cast<unsigned>((K + kCols - 1) / kCols));
+  with_order(p, [&](auto P_) {
+    m2m_kernel<decltype(P_)::value><<<grid, kShiftThreads, sizeof(float) * 4 * static_cast<size_t>(n) * kPitch, s>>>(
+        M, coef + static_cast<size_t>(parent_level + 1) * 8 * n, K, parent_level, parents, nP);
+  });
+}
+
+void launch_l2l(float *L, const float *coef, int n, int p, int K, int child_level, cudaStream_t s,
+                const ReducedLocals *red) {
+  const long long parents = 1LL << (3 * (child_level - 1));
+  const int nP = parents_per_cta(K);
+  const dim3 grid(static_cast<unsigned>((parents + nP - 1) / nP), static_cast<unsigned>((K + kCols - 1) / kCols), 4);
+  const float *level_coef = coef + static_cast<size_t>(child_level) * 8 * n;
+  const size_t planes = 2 * static_cast<size_t>(n), reduced = 2 * static_cast<size_t>(p + 1) * (p + 1);
+  with_order(p, [&](auto P_) {
+    constexpr int P = decltype(P_)::value;
+    if (red != nullptr)
+      l2l_kernel<P, true><<<grid, kShiftThreads, sizeof(float) * kPitch * (planes + reduced), s>>>(
+          L, level_coef, K, child_level, parents, nP, *red);
+    else
+      l2l_kernel<P, false><<<grid, kShiftThreads, sizeof(float) * kPitch * planes, s>>>(
+          L, level_coef, K, child_level, parents, nP, ReducedLocals{});
+  });
+}
+
+void configure_shift_kernels(int p, size_t max_smem) {
+  with_order(p, [&](auto P_) {
+    constexpr int P = decltype(P_)::value;
+    allow_dynamic_smem(m2m_kernel<P>, max_smem);
+    allow_dynamic_smem(l2l_kernel<P, false>, max_smem);
+    allow_dynamic_smem(l2l_kernel<P, true>, max_smem);
+    prefer_max_shared_carveout(l2l_kernel<P, false>); // run beside the co-resident near field
+    prefer_max_shared_carveout(l2l_kernel<P, true>);
+  });
+}
+
+} // namespace cdfmm_b200

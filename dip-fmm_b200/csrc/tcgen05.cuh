@@ -104,6 +104,29 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return d;
 }
 
+// K-major rows of 64 bytes with the 64-byte swizzle of a tiled TMA load
+// (16-byte units XORed with bits of the row; 8-row groups of 512 bytes,
+// 512-byte aligned); a 32-byte k-step advances the start address.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((addr >> 4) & 0x3fffu);
+  d |= static_cast<uint64_t>(1u) << 16;
+  d |= static_cast<uint64_t>(512u >> 4) << 32;
+  d |= static_cast<uint64_t>(1u) << 46; // version
+  d |= static_cast<uint64_t>(4u) << 61; // SWIZZLE_64B
+  return d;
+}
+
+// Tiled TMA load of a 4-D box at coordinates (x, y, z, w), x fastest; the part
+// outside the tensor reads zero.
+__device__ __forceinline__ void tma_load_4d(void *smem_dst, const void *map, int x, int y, int z, int w,
+                                            uint64_t *bar) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, "
+               "%5, %6}], [%2];" ::"r"(smem_u32(smem_dst)),
+               "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
+
 // Instruction descriptors, D = F32, K-major A and B, M = 128:
 // kind::f16 with A = B = BF16, and kind::tf32.
 __host__ __device__ constexpr uint32_t instr_desc_bf16(int n) {

@@ -1,0 +1,68 @@
+"""The far field over the edges of its tiles: states around the row boxes of
+the tensor-core M2L (one state, odd counts, the switch between whole-parent and
+(parent, state) rows at 32, partial last tiles, 128) and the state blocks of
+the shifts, orders with one and two operator column groups, trees of one M2L
+level and of several.
+
+The local expansions of every level are compared with the FP64 oracle FMM's
+potential and field on targets far from every source of their own leaf's
+neighbourhood -- here with the near field exact on both sides, the difference
+of the two evaluations is the far field's.
+"""
+
+import numpy as np
+import pytest
+
+import cdfmm_b200
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+# Split BF16 drops lo x lo, 2^-16 of each product; summed over the 189 offsets
+# with random signs that stays below 2^-16 of the far field, itself at most the
+# total on a lattice whose dipoles have no close pairs: 1.5e-5, doubled for the
+# FP32 shifts, near field and leaf sums.
+REL = 3e-5
+
+
+@pytest.mark.parametrize("order,depth,K", [(1, 2, 1), (4, 3, 1), (5, 3, 3), (3, 2, 7), (6, 3, 31), (2, 3, 32),
+                                            (4, 2, 33), (3, 3, 40), (7, 2, 5), (8, 3, 12), (5, 2, 100), (9, 2, 65),
+                                            (3, 2, 128), (0, 2, 4)])
+def test_states_and_orders_over_tile_edges(order, depth, K):
+    rng = np.random.default_rng(100 * order + K)
+    side = 2 << depth
+    g = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    x = (g + 0.5 + rng.uniform(-0.1, 0.1, g.shape)) / side
+    n = len(x)
+    m = rng.normal(size=(K, n, 3)).astype(np.float32)
+    plan = cdfmm_b200.DevicePlan.from_points(x, order, depth, max_states=K)
+    out = plan.evaluate(m, output="both")
+    assert plan.stats()["m2l_mode_resolved"] == cdfmm_b200.M2L_BF16X3
+    plan.close()
+    for k in sorted({0, K // 2, K - 1}):
+        ref = oracle.fmm(x, x, m[k].astype(np.float64), order, depth, identities=np.arange(n))
+        assert oracle.rel_l2(out["H"][k], ref["H"]) < REL
+        assert oracle.rel_l2(out["phi"][k], ref["phi"]) < REL
+
+
+@pytest.mark.parametrize("order,K", [(3, 2), (6, 1), (6, 48), (8, 5), (10, 3)])
+def test_fp32_m2l_with_separable_shifts(order, K):
+    # the FP32 M2L leaves its locals in place and the L2L adds to them
+    rng = np.random.default_rng(order + K)
+    depth, n = 3, 3000
+    x = rng.uniform(0, 1, (n, 3))
+    m = rng.normal(size=(K, n, 3)).astype(np.float32)
+    plan = cdfmm_b200.DevicePlan.from_points(x, order, depth, max_states=K, m2l_mode=cdfmm_b200.M2L_FP32)
+    out = plan.evaluate(m, output="both")
+    M = plan.read_expansions("multipole", K - 1)
+    L = plan.read_expansions("local", K - 1)
+    plan.close()
+    ref = oracle.fmm(x, x, m[K - 1].astype(np.float64), order, depth, identities=np.arange(n))
+    assert oracle.rel_l2(out["phi"][K - 1], ref["phi"]) < REL
+    assert np.isfinite(M).all() and np.isfinite(L).all()
+    # multipoles of the root: the sum over all sources of m_c d^(alpha - e_c), |alpha| = 1 -> -sum m_c
+    lo, hi = x.min(axis=0), x.max(axis=0)
+    scale = (hi - lo).max()
+    np.testing.assert_allclose(M[0][1:4][::-1], -m[K - 1].astype(np.float64).sum(axis=0) / scale ** 3, rtol=0,
+                               atol=2e-6 * np.abs(m[K - 1]).sum() / scale ** 3)
