@@ -24,13 +24,12 @@ inline int moment_row(int K) { return moments_paired(K) ? (K + 1) & ~1 : K; }
 // even in the paired layout.
 void launch_gather_moments(const void *user, int dtype, const int *inv, int ns, int K,
                            double scale, float4 *mom, cudaStream_t s, bool paired, int k0 = 0, int k_total = -1);
-size_t p2m_smem_bytes(int n, int p, int K, int chunk);
 // size != nullptr: uniformly magnetised cuboid sources, the monomials
 // averaged over each source's cuboid (normalised side lengths, size[j] per
 // source when size_step is 1, size[0] for all when 0).
-void launch_p2m(const float4 *src_rel, const float4 *mom, const int *src_off, const int8_t *basis,
-                float *M, int n, int p, int K, int depth, int chunk, cudaStream_t s,
-                const float4 *size = nullptr, int size_step = 0);
+void launch_p2m(const float4 *src_rel, const float4 *mom, const int *src_off, float *M, int p, int K, int depth,
+                cudaStream_t s, const float4 *size = nullptr, int size_step = 0);
+void configure_leaf_kernels(int p, size_t max_smem);
 // M2M of one parent level and L2L of one child level (separable shifts,
 // shift_kernels.cu); coef = the plan's [(depth + 1) * 8][n] shift table.
 void launch_m2m(float *M, const float *coef, int n, int p, int K, int parent_level, cudaStream_t s);
@@ -45,7 +44,6 @@ struct ReducedLocals {
 void launch_l2l(float *L, const float *coef, int n, int p, int K, int child_level, cudaStream_t s,
                 const ReducedLocals *red = nullptr);
 void configure_shift_kernels(int p, size_t max_smem);
-size_t l2p_smem_bytes(int n, int p, int Kb);
 // L2P + combine; K >= 4 writes the sorted results over `near` and then unsorts
 // them to user order (2 launches), K < 4 writes user order directly.  A state
 // range [k_begin, k_end) (K >= 4 only; default all K) processes those states
@@ -53,10 +51,11 @@ size_t l2p_smem_bytes(int n, int p, int Kb);
 // field yet: L2P writes the far field alone there, and a later P2P in
 // accumulate mode adds the near field; unsort = false leaves the results
 // sorted (launch_unsort does that part).
-void launch_l2p(const float *L, const float4 *tgt_rel, const int *tgt_off, const int *tgt_perm, const int *tgt_inv,
-                float4 *near, const int8_t *basis, int n, int p, int K, int nt, int depth, unsigned output,
-                int layout, float phi_scale, float *field, float *potential, cudaStream_t s, int k_begin = 0,
-                int k_end = -1, int k_near_end = -1, bool unsort = true);
+// Returns the launch count.
+int launch_l2p(const float *L, const float4 *tgt_rel, const int *tgt_off, const int *tgt_perm, const int *tgt_inv,
+               float4 *near, int p, int K, int nt, int depth, unsigned output, int layout, float phi_scale,
+               float *field, float *potential, cudaStream_t s, int k_begin = 0, int k_end = -1,
+               int k_near_end = -1, bool unsort = true);
 // Sorted combined results (near, K states per target) of states
 // [k_begin, k_end) -> user order (the second launch of launch_l2p).
 void launch_unsort(const float4 *res, const int *tgt_inv, int nt, int K, unsigned output, int layout, float *field,

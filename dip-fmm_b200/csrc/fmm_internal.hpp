@@ -214,7 +214,6 @@ struct cdfmm_b200_plan {
   int4 *m2l_tiles = nullptr;   // SIMT M2L work tiles (level, class, packed parent origin)
   int n_tiles = 0;
   int8_t *basis = nullptr;     // [n][4] ax, ay, az, degree
-  int p2m_chunk = 64;
   int last_K = 0;              // states whose expansions M, L hold (from state exp_state0)
   int exp_state0 = 0;
 

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <type_traits>
 
 namespace cdfmm_b200 {
 
@@ -81,7 +82,25 @@ __host__ __device__ inline void demorton3(uint32_t m, int &x, int &y, int &z) {
   z = static_cast<int>(undilate3(m >> 2));
 }
 
+// Calls f with the expansion order 0 <= p <= 10 as a compile-time constant.
+template <int P = 0, class F> inline void with_order(int p, F f) {
+  if constexpr (P <= 10) {
+    if (p == P)
+      f(std::integral_constant<int, P>{});
+    else
+      with_order<P + 1>(p, f);
+  }
+}
+
 #ifdef __CUDACC__
+// Calls f(integral_constant R0) for R0 = 0, 32, 64, ... below N.
+template <int N, int R0 = 0, class F> __device__ __forceinline__ void static_rows(F f) {
+  if constexpr (R0 < N) {
+    f(std::integral_constant<int, R0>{});
+    static_rows<N, R0 + 32>(f);
+  }
+}
+
 // 16-byte (and 4-byte) asynchronous global -> shared copy (bypasses registers, so many
 // copies of one thread are in flight at once), its commit and wait.
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {

@@ -601,12 +601,9 @@ static void finish_plan(cdfmm_b200_plan *plan, int m2l_mode) {
   const size_t smem = device_smem_optin(plan->device);
   configure_far_kernels(smem);
   configure_shift_kernels(plan->p, smem);
+  configure_leaf_kernels(plan->p, smem);
   configure_m2l_simt(smem);
   configure_p2p(smem);
-  plan->p2m_chunk = 64;
-  while (plan->p2m_chunk > 8 && p2m_smem_bytes(n, plan->p, static_cast<int>(K), plan->p2m_chunk) > smem) plan->p2m_chunk /= 2;
-  require(p2m_smem_bytes(n, plan->p, 4, plan->p2m_chunk) <= smem && l2p_smem_bytes(n, plan->p, 4) <= smem,
-          "order exceeds the shared-memory budget of one CTA");
   check(cudaDeviceSynchronize(), "plan upload");
   plan->error_flag = dalloc<int>(1, bytes);
   check(cudaMemset(plan->error_flag, 0, sizeof(int)), "cudaMemset");
@@ -1018,6 +1015,14 @@ int cdfmm_b200_set_self_indices(cdfmm_b200_plan *plan, const int32_t *sorted_sel
   }
 }
 
+// The tensor-core P2M (beside the tensor-core near field) pays for leaves of
+// many sources and many states: 64 per leaf, p = 6, K = 64, N = 262,144 0.28
+// against 0.59 ms for the register form; at 32 per leaf it is behind (N = 1M, K
+// = 64 1.31 against 1.11 ms), and with 16 states well behind (64 per leaf 0.25
+// against 0.10 ms).  On trees of at most 512 leaves either takes tens of
+// microseconds, and the tensor-core form stays for every state count.
+constexpr int kP2mTcLeafSources = 48, kP2mTcStates = 32, kP2mTcLeaves = 512;
+
 // Upward pass for K states whose sorted, scaled moments are in plan->mom:
 // P2M and M2M, leaving the multipoles in plan->M.  Returns the launch count.
 // With `ntc` (the tensor-core near field's moment blocks, packed for these
@@ -1026,11 +1031,13 @@ static int enqueue_upward(cdfmm_b200_plan *plan, int K, cudaStream_t s, bool tim
                           const NearTcLaunch *ntc = nullptr) {
   const int n = plan->n;
   int launches = 0;
-  if (ntc != nullptr && plan->p2m_tc_ok && !plan->cuboid_p2m && p2m_tc_supported(n, K))
+  if (ntc != nullptr && plan->p2m_tc_ok && !plan->cuboid_p2m && p2m_tc_supported(n, K) &&
+      static_cast<long long>(plan->ns) >= static_cast<long long>(kP2mTcLeafSources) * plan->n_leaves &&
+      (K >= kP2mTcStates || plan->n_leaves <= kP2mTcLeaves))
     launch_p2m_tc(*ntc, plan->basis, plan->M, n, plan->p, K, plan->depth, s);
   else
-    launch_p2m(plan->src_rel, plan->mom, plan->src_off, plan->basis, plan->M, n, plan->p, K, plan->depth,
-               plan->p2m_chunk, s, plan->cuboid_p2m ? plan->src_size : nullptr, plan->size_step);
+    launch_p2m(plan->src_rel, plan->mom, plan->src_off, plan->M, plan->p, K, plan->depth, s,
+               plan->cuboid_p2m ? plan->src_size : nullptr, plan->size_step);
   ++launches;
   if (timing) check(cudaEventRecord(plan->ev_t[2], s), "event");
   for (int level = plan->depth - 1; level >= 0; --level) {
@@ -1285,9 +1292,7 @@ static int enqueue_evaluation(cdfmm_b200_plan *plan, const void *moments, int dt
     check(cudaStreamWaitEvent(s, plan->ev_join, 0), "wait");
   }
   if (timing) check(cudaEventRecord(plan->ev_t[6], s), "event");
-  launch_l2p(plan->L, plan->tgt_rel, plan->tgt_off, plan->tgt_perm, plan->tgt_inv, plan->near, plan->basis, plan->n,
-             plan->p, K, plan->nt, plan->depth, output, layout, plan->phi_scale, field, potential, s);
-  launches += (K >= 4 && plan->nt > 0) ? 2 : 1;
+  launches += launch_l2p(plan->L, plan->tgt_rel, plan->tgt_off, plan->tgt_perm, plan->tgt_inv, plan->near, plan->p, K, plan->nt, plan->depth, output, layout, plan->phi_scale, field, potential, s);
   check(cudaGetLastError(), "kernel launch");
   if (timing) check(cudaEventRecord(plan->ev_t[7], s), "event");
   if (trace) check(cudaEventRecord(plan->ev_t[kTraceEnd], s), "event");
@@ -1314,8 +1319,7 @@ void cdfmm_b200_stacked_downward(cdfmm_b200_plan *plan, const cdfmm_b200_eval_ar
   for (int level = 2; level <= plan->depth; ++level)
     launch_l2l(plan->L, plan->l2l_coef, plan->n, plan->p, 1, level, s, &red);
   check(cudaStreamWaitEvent(s, plan->ev_join, 0), "wait");
-  launch_l2p(plan->L, plan->tgt_rel, plan->tgt_off, plan->tgt_perm, plan->tgt_inv, plan->near, plan->basis, plan->n,
-             plan->p, 1, plan->nt, plan->depth, a->output, a->layout, plan->phi_scale, a->field, a->potential, s);
+  launch_l2p(plan->L, plan->tgt_rel, plan->tgt_off, plan->tgt_perm, plan->tgt_inv, plan->near, plan->p, 1, plan->nt, plan->depth, a->output, a->layout, plan->phi_scale, a->field, a->potential, s);
   check(cdfmm_b200_collect_status(plan, s, plan->call_seq), "status kernel launch");
   check(cudaGetLastError(), "kernel launch");
   plan->last_m2l_tc = true;
@@ -1476,8 +1480,7 @@ int cdfmm_b200_evaluate(cdfmm_b200_plan *plan, const cdfmm_b200_eval_args *a) {
       launches += enqueue_far(plan, K, s, false);
       // one L2P for all K states: combined with the near field of the early
       // parts, far field alone for the later ones
-      launch_l2p(plan->L, plan->tgt_rel, plan->tgt_off, plan->tgt_perm, plan->tgt_inv, plan->near, plan->basis,
-                 plan->n, plan->p, K, plan->nt, plan->depth, a->output, a->layout, plan->phi_scale,
+      launch_l2p(plan->L, plan->tgt_rel, plan->tgt_off, plan->tgt_perm, plan->tgt_inv, plan->near, plan->p, K, plan->nt, plan->depth, a->output, a->layout, plan->phi_scale,
                  reinterpret_cast<float *>(field), reinterpret_cast<float *>(potential), s, 0, K, bounds[early], false);
       ++launches;
       for (int j = 0; j < early; ++j) finish_part(j);

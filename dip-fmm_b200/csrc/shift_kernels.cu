@@ -370,16 +370,6 @@ __global__ void __launch_bounds__(kShiftThreads, P <= 6 ? 4 : P <= 8 ? 3 : 2)
 // Whole parents per CTA.
 int parents_per_cta(int K) { return K >= kCols ? 1 : kCols / K; }
 
-// Calls f with the order as a compile-time constant.
-template <int P = 0, class F> void with_order(int p, F f) {
-  if constexpr (P <= 10) {
-    if (p == P)
-      f(std::integral_constant<int, P>{});
-    else
-      with_order<P + 1>(p, f);
-  }
-}
-
 } // namespace
 
 void launch_m2m(float *M, const float *coef, int n, int p, int K, int parent_level, cudaStream_t s) {
