@@ -43,6 +43,13 @@ namespace {
 
 using namespace tc;
 
+// 1 / sqrt(x), a subnormal x read as zero (see near_kernels.cu).
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 constexpr int kNgThreads = 192;       // warps 0-3 weights + epilogue, 4 copies, 5 MMA
 constexpr uint32_t kNgTmemCols = 256; // two CTAs per SM
 constexpr int kNgRows = 3 * kNearGradSources; // 48 accumulator columns per chunk
@@ -140,7 +147,7 @@ __device__ __forceinline__ void chunk_grad_any(int c, const float4 *p16, float t
     const float4 p = p16[q];
     const float rx = tx - p.x, ry = ty - p.y, rz = tz - p.z;
     const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-    const float rinv = __float_as_int(p.w) == self ? 0.0F : rsqrtf(r2);
+    const float rinv = __float_as_int(p.w) == self ? 0.0F : rsqrt_ftz(r2);
     const float r2inv = rinv * rinv;
     const float f5 = 3.0F * r2inv * r2inv * rinv;
     const float f7 = 5.0F * f5 * r2inv;
@@ -163,7 +170,7 @@ __device__ __forceinline__ void chunk_grad(const float4 *p16, float tx, float ty
     const float4 p = p16[q];
     const float rx = tx - p.x, ry = ty - p.y, rz = tz - p.z;
     const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-    const float rinv = __float_as_int(p.w) == self ? 0.0F : rsqrtf(r2);
+    const float rinv = __float_as_int(p.w) == self ? 0.0F : rsqrt_ftz(r2);
     const float r2inv = rinv * rinv;
     const float f5 = 3.0F * r2inv * r2inv * rinv;
     const float f7 = 5.0F * f5 * r2inv;

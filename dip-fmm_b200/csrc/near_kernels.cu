@@ -74,15 +74,44 @@ __device__ void build_neighbours(Neighbours &nb, int leaf, int depth, const int 
   }
 }
 
-// Stages sources [g0, g0 + cnt) of the flattened neighbourhood: position
-// relative to the target leaf centre and the sorted source index in .w.
-__device__ inline void stage_source(const Neighbours &nb, int g, const float4 *src_rel,
-                                    float4 &pos, int &j) {
-  int b = 0;
+// Source g of the flattened neighbourhood: position relative to the target
+// leaf centre and the sorted source index in .w.  b: its neighbour, searched
+// from the value given (a thread that stages rising g passes it on).
+__device__ inline void stage_source_from(const Neighbours &nb, int g, const float4 *src_rel, float4 &pos, int &j,
+                                         int &b) {
   while (b + 1 < nb.count && nb.prefix[b + 1] <= g) ++b;
   j = nb.begin[b] + (g - nb.prefix[b]);
   const float4 d = src_rel[j];
   pos = make_float4(d.x + nb.sx[b], d.y + nb.sy[b], d.z + nb.sz[b], __int_as_float(j));
+}
+__device__ inline void stage_source(const Neighbours &nb, int g, const float4 *src_rel, float4 &pos, int &j) {
+  int b = 0;
+  stage_source_from(nb, g, src_rel, pos, j, b);
+}
+
+// 1 / sqrt(x) with a subnormal x read as zero: the pair kernels cube it, and
+// 1 / x^(3/2) of a subnormal overflows either way; without the subnormal case
+// it is one instruction (rsqrtf adds a compare and two scalings per pair).
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Sums v[0..15] over the warp's lanes: lane l returns the sum of v[l >> 1].
+// Each step halves the values a lane carries: 16 shuffles in all, where 16
+// butterflies take 80 (the same additions in the same order).
+__device__ __forceinline__ float sum16(float (&v)[16], int lane) {
+#pragma unroll
+  for (int o = 16, h = 8; h >= 1; o >>= 1, h >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < h; ++j) {
+      const float keep = up ? v[j + h] : v[j], send = up ? v[j] : v[j + h];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
 // Close pairs.  Positions are kept in FP32 relative to their leaf centre,
@@ -113,7 +142,7 @@ __device__ __forceinline__ void pair_k1_x2(const float2 &ntx, const float2 &nty,
   const float2 dy = __fadd2_rn(make_float2(pxy.z, pxy.w), nty);
   const float2 dz = __fadd2_rn(make_float2(pzj.x, pzj.y), ntz);
   const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-  float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+  float2 rinv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
   if (SELF) {
     rinv.x = __float_as_int(pzj.z) == self ? 0.0F : rinv.x;
     rinv.y = __float_as_int(pzj.w) == self ? 0.0F : rinv.y;
@@ -156,7 +185,11 @@ __device__ __forceinline__ void k1_segment(const float2 (&nt)[4][3], const int (
 // j1 | mx0 mx1 my0 my1 | mz0 mz1; an odd chunk is padded with a zero moment
 // 1e18 away), so each lane reads two sources' operands ready for packed
 // FP32x2 arithmetic; each warp owns 4 targets at a time, lanes stride over
-// the staged pairs and the partial sums are combined with warp shuffles.
+// the staged pairs and the 16 partial sums are combined by sum16.  Bound: the
+// FMA pipes (19-20 operations per pair).  Measured (before: rsqrtf, 16
+// butterflies per 4 targets, each staged source's neighbour searched from the
+// first): N = 1M, 32 per leaf, both outputs 1.18 -> 0.95 ms (8.5e8 pairs); 48
+// clustered problems, 5.3e10 pairs 46.0 -> 39.1 ms.
 // Only the staged positions of the sources between the lowest and highest
 // self source of the leaf's targets are compared against the self indices
 // (the own leaf's, when sources and targets are the same points).
@@ -211,14 +244,15 @@ __global__ void __launch_bounds__(128) p2p_k1_kernel(const float4 *__restrict__ 
       const int sn = min(kK1Chunk, total - sc);
       const int np = (sn + 1) / 2;
       __syncthreads();
+      int nb_at = 0;
       for (int q = threadIdx.x; q < np; q += blockDim.x) {
         float4 p0, p1 = make_float4(1.0e18F, 1.0e18F, 1.0e18F, __int_as_float(-1));
         float4 m0, m1 = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
         int j;
-        stage_source(nb, sc + 2 * q, src_rel, p0, j);
+        stage_source_from(nb, sc + 2 * q, src_rel, p0, j, nb_at);
         m0 = mom[j];
         if (2 * q + 1 < sn) {
-          stage_source(nb, sc + 2 * q + 1, src_rel, p1, j);
+          stage_source_from(nb, sc + 2 * q + 1, src_rel, p1, j, nb_at);
           m1 = mom[j];
         }
         sPxy[q] = make_float4(p0.x, p1.x, p0.y, p1.y);
@@ -248,28 +282,15 @@ __global__ void __launch_bounds__(128) p2p_k1_kernel(const float4 *__restrict__ 
         k1_segment<PHI, false>(nt, self, sPxy, sPzj, sMxy, sMz, 0, pa, lane, acc2);
         k1_segment<PHI, true>(nt, self, sPxy, sPzj, sMxy, sMz, pa, pb, lane, acc2);
         k1_segment<PHI, false>(nt, self, sPxy, sPzj, sMxy, sMz, pb, np, lane, acc2);
-        float acc[4][4];
+        float acc[16];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            acc[u][c] = -(acc2[u][c].x + acc2[u][c].y); // phi = -P, H = -G
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[u][c] += __shfl_xor_sync(0xffffffffu, acc[u][c], o);
-          }
-        if (lane == 0) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (tb + u < tn) {
-              float4 a = sAcc[tb + u];
-              a.x += acc[u][0];
-              a.y += acc[u][1];
-              a.z += acc[u][2];
-              a.w += acc[u][3];
-              sAcc[tb + u] = a;
-            }
-          }
-        }
+          for (int c = 0; c < 4; ++c) acc[4 * u + c] = -(acc2[u][c].x + acc2[u][c].y); // phi = -P, H = -G
+        const float sum = sum16(acc, lane);
+        const int v = lane >> 1;
+        if ((lane & 1) == 0 && tb + (v >> 2) < tn)
+          reinterpret_cast<float *>(sAcc + tb + (v >> 2))[v & 3] += sum;
       }
     }
     __syncthreads();
@@ -346,7 +367,7 @@ __device__ __forceinline__ void p2p_kb_chunk(const float4 &ti, int self, const f
     const float dx = ti.x - s.x, dy = ti.y - s.y, dz = ti.z - s.z;
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     const bool is_self = __float_as_int(s.w) == self;
-    const float rinv = is_self ? 0.0F : rsqrtf(r2);
+    const float rinv = is_self ? 0.0F : rsqrt_ftz(r2);
     const float v = rinv * rinv * rinv;
     const float f = 3.0F * v * rinv * rinv;
     const float ux = f * dx, uy = f * dy, uz = f * dz;
@@ -382,7 +403,7 @@ __device__ __forceinline__ void p2p_kb_chunk_x2(const float4 &ti, int self_q, co
     const float4 s = sPos[q];
     const float dx = ti.x - s.x, dy = ti.y - s.y, dz = ti.z - s.z;
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    const float rinv = q == self_q ? 0.0F : rsqrtf(r2);
+    const float rinv = q == self_q ? 0.0F : rsqrt_ftz(r2);
     const float v = rinv * rinv * rinv;
     const float f = 3.0F * v * rinv * rinv;
     const float w = r2 * (1.0F / 3.0F);
@@ -423,7 +444,7 @@ __device__ __forceinline__ void p2p_grad_chunk(const float4 &ti, int self, const
     const float dx = ti.x - s.x, dy = ti.y - s.y, dz = ti.z - s.z;
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     const bool is_self = __float_as_int(s.w) == self;
-    const float rinv = is_self ? 0.0F : rsqrtf(r2);
+    const float rinv = is_self ? 0.0F : rsqrt_ftz(r2);
     const float r2inv = rinv * rinv;
     const float f5 = 3.0F * r2inv * r2inv * rinv;
     const float f7 = 5.0F * f5 * r2inv;
@@ -944,7 +965,7 @@ __device__ __forceinline__ float3 moment_of(const float4 *mom, int j, int K, int
 // Pair field at r (= target - source) for moment m: (phi, H) times 4 pi.
 __device__ __forceinline__ float4 pair_field(float rx, float ry, float rz, float3 m) {
   const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-  const float rinv = rsqrtf(r2);
+  const float rinv = rsqrt_ftz(r2);
   const float v = rinv * rinv * rinv;
   const float mr = fmaf(m.x, rx, fmaf(m.y, ry, m.z * rz));
   const float f = 3.0F * mr * v * rinv * rinv;
@@ -953,7 +974,7 @@ __device__ __forceinline__ float4 pair_field(float rx, float ry, float rz, float
 // Position gradient of w . H (times 4 pi) at r for moment m.
 __device__ __forceinline__ float3 pair_grad(float rx, float ry, float rz, float3 m, float3 w) {
   const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-  const float rinv = rsqrtf(r2);
+  const float rinv = rsqrt_ftz(r2);
   const float r2inv = rinv * rinv;
   const float f5 = 3.0F * r2inv * r2inv * rinv, f7 = 5.0F * f5 * r2inv;
   const float a = fmaf(m.x, rx, fmaf(m.y, ry, m.z * rz)), b = fmaf(w.x, rx, fmaf(w.y, ry, w.z * rz));

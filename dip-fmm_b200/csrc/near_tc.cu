@@ -61,6 +61,13 @@ namespace {
 
 using namespace tc;
 
+// 1 / sqrt(x), a subnormal x read as zero (see near_kernels.cu).
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // Warp roles: 0-3 pair tensors (warp c: component c); 4 copies; 5 MMA issue
 // and tensor-memory allocation; 6-9 accumulator drains and the epilogue.
 // Pair-tensor warpgroups (chunks are dealt round robin): one with two
@@ -178,7 +185,7 @@ __device__ __forceinline__ void chunk_tensors(const float4 *p8, float ntx, float
     const float2 dy = __fadd2_rn(make_float2(p0.y, p1.y), make_float2(nty, nty));
     const float2 dz = __fadd2_rn(make_float2(p0.z, p1.z), make_float2(ntz, ntz));
     const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-    float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+    float2 rinv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
     rinv.x = __float_as_int(p0.w) == self ? 0.0F : rinv.x;
     rinv.y = __float_as_int(p1.w) == self ? 0.0F : rinv.y;
     const float2 rinv2 = __fmul2_rn(rinv, rinv);
