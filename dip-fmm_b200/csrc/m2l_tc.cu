@@ -70,7 +70,7 @@ constexpr int kTcThreads = 128;
 constexpr uint32_t kWaitLimit = kTcWaitLimit; // ~2 s with the back-off below
 constexpr int kChunk = 16;                    // alphas per pipeline stage (one MMA k-step)
 constexpr uint32_t kABytes = kM2lRows * kChunk * 4u; // rows of [hi 16 | lo 16] BF16: 64 bytes each
-constexpr int kSlab = 32;                     // accumulator columns staged at a time by the epilogue
+constexpr int kSlab = 128;                    // accumulator columns staged at a time by the epilogue
 constexpr int kSlabPitch = kSlab + 1;
 
 using tc::bulk_g2s;
@@ -298,9 +298,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) m2l_tc_kernel(const __grid_cons
   // Epilogue: warp w owns TMEM lanes 32w..32w+31, one row per thread.  Column
   // q of the group is local (class, beta) = (q / n_out, q % n_out), which is
   // float q * K + state of the parent's rows of R.  Many states: consecutive
-  // lanes are consecutive states, stored directly; few: 32 columns at a time
+  // lanes are consecutive states, stored directly; few: 128 columns at a time
   // go through the idle stage memory, so that a warp stores the contiguous
-  // 32 K floats of one parent.
+  // floats of one parent.
   float *R = args.R + split * args.split_stride;
   const int n_cols = (8 / args.groups) * args.n_out;
   const uint32_t tlane = tmem + (static_cast<uint32_t>(warp * 32) << 16);
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) m2l_tc_kernel(const __grid_cons
   } else {
     float *slab = reinterpret_cast<float *>(smem);
     const int segs = (lv.bx / K) * lv.by * lv.bz;
-    const uint32_t magic = 65536u / static_cast<uint32_t>(K) + 1u; // e / K = e * magic >> 16 for e < 1024, K < 32
+    const uint32_t magic = (1u << 20) / static_cast<uint32_t>(K) + 1u; // e / K = e * magic >> 20 for e < 4096, K < 32
     for (int c0 = 0; c0 < args.cols; c0 += kSlab) {
       for (int h = 0; h < kSlab && c0 + h < args.cols; h += 16) {
         float v[16];
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) m2l_tc_kernel(const __grid_cons
         if (base < 0) continue;
         float *dst = R + base + static_cast<long long>(c0) * K;
         for (int e = lane; e < run; e += 32) {
-          const int c = static_cast<int>((static_cast<uint32_t>(e) * magic) >> 16);
+          const int c = static_cast<int>((static_cast<uint32_t>(e) * magic) >> 20);
           dst[e] = slab[(q * K + e - c * K) * kSlabPitch + c];
         }
       }

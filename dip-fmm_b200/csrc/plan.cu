@@ -134,6 +134,7 @@ void free_plan(cdfmm_b200_plan *p) {
   if (p->near_stream) cudaStreamDestroy(p->near_stream);
   if (p->far_stream) cudaStreamDestroy(p->far_stream);
   if (p->ev_far) cudaEventDestroy(p->ev_far);
+  if (p->ev_up) cudaEventDestroy(p->ev_up);
   if (p->stream) cudaStreamDestroy(p->stream);
   delete p;
 }
@@ -354,6 +355,7 @@ static cdfmm_b200_plan *new_plan(int ns, int nt, int order, int depth, int max_s
       check(cudaDeviceGetStreamPriorityRange(&least, &greatest), "stream priorities");
       check(cudaStreamCreateWithPriority(&plan->far_stream, cudaStreamNonBlocking, greatest), "cudaStreamCreate");
       check(cudaEventCreateWithFlags(&plan->ev_far, cudaEventDisableTiming), "cudaEventCreate");
+      check(cudaEventCreateWithFlags(&plan->ev_up, cudaEventDisableTiming), "cudaEventCreate");
     }
     check(cudaStreamCreateWithFlags(&plan->io_in, cudaStreamNonBlocking), "cudaStreamCreate");
     check(cudaStreamCreateWithFlags(&plan->io_out, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -1024,11 +1026,11 @@ int cdfmm_b200_set_self_indices(cdfmm_b200_plan *plan, const int32_t *sorted_sel
 constexpr int kP2mTcLeafSources = 48, kP2mTcStates = 32, kP2mTcLeaves = 512;
 
 // Upward pass for K states whose sorted, scaled moments are in plan->mom:
-// P2M and M2M, leaving the multipoles in plan->M.  Returns the launch count.
-// With `ntc` (the tensor-core near field's moment blocks, packed for these
+// P2M and M2M down to parent level `top`, leaving the multipoles in plan->M.
+// Returns the launch count.  With `ntc` (the tensor-core near field's moment blocks, packed for these
 // K states) the leaf multipoles run on the tensor cores where they can.
 static int enqueue_upward(cdfmm_b200_plan *plan, int K, cudaStream_t s, bool timing,
-                          const NearTcLaunch *ntc = nullptr) {
+                          const NearTcLaunch *ntc = nullptr, int top = 0) {
   const int n = plan->n;
   int launches = 0;
   if (ntc != nullptr && plan->p2m_tc_ok && !plan->cuboid_p2m && p2m_tc_supported(n, K) &&
@@ -1040,7 +1042,7 @@ static int enqueue_upward(cdfmm_b200_plan *plan, int K, cudaStream_t s, bool tim
                plan->cuboid_p2m ? plan->src_size : nullptr, plan->size_step);
   ++launches;
   if (timing) check(cudaEventRecord(plan->ev_t[2], s), "event");
-  for (int level = plan->depth - 1; level >= 0; --level) {
+  for (int level = plan->depth - 1; level >= top; --level) {
     launch_m2m(plan->M, plan->m2m_coef, n, plan->p, K, level, s);
     ++launches;
   }
@@ -1271,15 +1273,30 @@ static int enqueue_evaluation(cdfmm_b200_plan *plan, const void *moments, int dt
   if (timing) check(cudaEventRecord(plan->ev_t[9], ns), "event");
   if (trace) check(cudaEventRecord(plan->ev_t[kTraceP2pEnd], ns), "event");
   if (timing) check(cudaEventRecord(plan->ev_t[1], s), "event");
-  if (!timing) check(cudaEventRecord(plan->ev_join, ns), "event");
 
   // far field
   if (corun) {
+    check(cudaEventRecord(plan->ev_join, ns), "event");
     if (trace) check(cudaEventRecord(plan->ev_t[kTraceM2lBegin], fs), "event");
     launches += enqueue_downward(plan, K, fs, false, true);
   } else {
     if (trace) check(cudaEventRecord(plan->ev_t[kTraceFarBegin], fs), "event");
-    launches += enqueue_upward(plan, K, fs, timing, near_tc ? &near_tc_args : nullptr);
+    // The multipoles of levels 0 and 1, which no M2L reads, are formed on the
+    // near stream, off the far field's chain of launches (a level is 6-9 us
+    // however small).
+    const int top = timing ? 0 : std::min(plan->depth, 2);
+    launches += enqueue_upward(plan, K, fs, timing, near_tc ? &near_tc_args : nullptr, top);
+    if (!timing) {
+      if (top > 0) {
+        check(cudaEventRecord(plan->ev_up, fs), "event");
+        check(cudaStreamWaitEvent(ns, plan->ev_up, 0), "wait");
+        for (int level = top - 1; level >= 0; --level) {
+          launch_m2m(plan->M, plan->m2m_coef, plan->n, plan->p, K, level, ns);
+          ++launches;
+        }
+      }
+      check(cudaEventRecord(plan->ev_join, ns), "event");
+    }
     if (trace) check(cudaEventRecord(plan->ev_t[kTraceM2lBegin], fs), "event");
     launches += enqueue_downward(plan, K, fs, timing);
   }

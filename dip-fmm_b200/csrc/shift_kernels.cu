@@ -246,13 +246,16 @@ __global__ void __launch_bounds__(kShiftThreads, P <= 6 ? 4 : P <= 8 ? 3 : 2)
     l2l_kernel(float *__restrict__ L, const float *__restrict__ coef, int K, int child_level, long long n_parents,
                int nP, const ReducedLocals red) {
   constexpr int n = (P + 1) * (P + 2) * (P + 3) / 6, n_out = (P + 1) * (P + 1);
-  extern __shared__ float sh[]; // two planes [n][kPitch], reduced locals of the two z children [2][n_out][kPitch]
+  // a plane [n][kPitch] (the x and y shifts work in place, a line at a time),
+  // the reduced locals of the two z children [2][n_out][kPitch], and (K <= 32)
+  // a second plane for the + child's locals
+  extern __shared__ float sh[];
   const Columns col = columns(n_parents, nP, K);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int xy = blockIdx.z;
   const float *row = coef + (4 + xy) * n; // class (x, y, +z)
   const bool shifted = !EXPAND || child_level > 2; // locals of levels 0 and 1 are zero
-  float *sA = sh, *sB = sh + n * kPitch, *sR = sB + n * kPitch;
+  float *sA = sh, *sR = sA + n * kPitch, *sB = sR + (EXPAND ? 2 * n_out * kPitch : 0);
   const long long child0 = level_offset_d(child_level) + col.parent0 * 8 + xy; // -z child; +z is 4 further
   const long long per4 = 4LL * n * K;
   if constexpr (EXPAND) {
@@ -298,7 +301,7 @@ __global__ void __launch_bounds__(kShiftThreads, P <= 6 ? 4 : P <= 8 ? 3 : 2)
       float v[m];
 #pragma unroll
       for (int i = 0; i < m; ++i) v[i] = sA[line_rank<0>(u, w, i) * kPitch + lane];
-      shift(M_, v, [&](int i, float x) { sB[line_rank<0>(u, w, i) * kPitch + lane] = x; });
+      shift(M_, v, [&](int i, float x) { sA[line_rank<0>(u, w, i) * kPitch + lane] = x; });
     });
     axis_coefficients<1, P>(row, c);
     __syncthreads();
@@ -306,7 +309,7 @@ __global__ void __launch_bounds__(kShiftThreads, P <= 6 ? 4 : P <= 8 ? 3 : 2)
       constexpr int u = decltype(U_)::value, w = decltype(W_)::value, m = decltype(M_)::value;
       float v[m];
 #pragma unroll
-      for (int i = 0; i < m; ++i) v[i] = sB[line_rank<1>(u, w, i) * kPitch + lane];
+      for (int i = 0; i < m; ++i) v[i] = sA[line_rank<1>(u, w, i) * kPitch + lane];
       shift(M_, v, [&](int i, float x) { sA[line_rank<1>(u, w, i) * kPitch + lane] = x; });
     });
   }
@@ -388,7 +391,7 @@ void launch_l2l(float *L, const float *coef, int n, int p, int K, int child_leve
   const int nP = parents_per_cta(K);
   const dim3 grid(static_cast<unsigned>((parents + nP - 1) / nP), static_cast<unsigned>((K + kCols - 1) / kCols), 4);
   const float *level_coef = coef + static_cast<size_t>(child_level) * 8 * n;
-  const size_t planes = 2 * static_cast<size_t>(n), reduced = 2 * static_cast<size_t>(p + 1) * (p + 1);
+  const size_t planes = (K > kCols ? 1 : 2) * static_cast<size_t>(n), reduced = 2 * static_cast<size_t>(p + 1) * (p + 1);
   with_order(p, [&](auto P_) {
     constexpr int P = decltype(P_)::value;
     if (red != nullptr)
