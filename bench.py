@@ -620,7 +620,7 @@ def b200_arm(args):
                    "m2l": ["auto", "fp32", "bf16x3"][st["m2l_mode_resolved"]],
                    "m2l_shape": {"accumulators_per_cta": st["m2l_tc_m_tiles"], "stages": st["m2l_tc_stages"],
                                  "fused_hi_lo_mma": bool(st["m2l_tc_fused"]),
-                                 "chosen_by": "autotuner"},
+                                 "chosen_by": "order"},
                    "l2": f"inputs larger than L2 ({dm.numel() * 4 / 2**20:.0f} MiB of moments per step)",
                    "parallelism": "replicas (independent states per GPU)" if world > 1 else "single GPU"},
         "rel_l2_H": rel_h, "rel_l2_phi": rel_phi,

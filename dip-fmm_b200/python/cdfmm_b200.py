@@ -453,8 +453,8 @@ class DevicePlan:
         return [(buf[3 * i], buf[3 * i + 1], bool(buf[3 * i + 2])) for i in range(n)]
 
     def set_m2l_shape(self, m_tiles, stages=0, fused=False):
-        """Pins one of m2l_shapes() (no autotuning, run-to-run identical
-        results); m_tiles = 0 returns to autotuning."""
+        """Pins one of m2l_shapes() (the first is the default);
+        m_tiles = 0 returns to the default."""
         _check(library().cdfmm_b200_set_m2l_shape(self._h, int(m_tiles), int(stages), 1 if fused else 0), self._h)
 
     def poll_status(self):

@@ -135,9 +135,9 @@ typedef struct cdfmm_b200_stats {
   int32_t m2l_mode_resolved;
   int32_t timing_enabled;
   int32_t m2l_tc_m_tiles;        /* tensor-core M2L shape last used: accumulators per CTA */
-  int32_t m2l_tc_stages;         /*   and pipeline stages (chosen by the autotuner in AUTO mode) */
+  int32_t m2l_tc_stages;         /*   and pipeline stages */
   int32_t backward_reused_forward; /* last backward reused the forward's moments and locals */
-  int32_t m2l_tc_fused;          /*   1: hi and lo translation tiles side by side in one wider MMA */
+  int32_t m2l_tc_fused;          /*   1: the hi x lo product in an accumulator of its own */
   double ms_gather, ms_p2m, ms_m2m, ms_m2l, ms_l2l, ms_l2p, ms_p2p, ms_total;
   /* Concurrent trace of the last evaluate (timing mode 2; ms from its start,
    * device events on the streams the stages ran on): near field begin / end,
@@ -333,8 +333,8 @@ int cdfmm_b200_backward(cdfmm_b200_plan *plan, const cdfmm_b200_backward_args *a
 /* Multi-geometry batches (no counterpart in the reference, which evaluates
  * one UniformFmm per call).  A batch evaluates `count` plans -- independent
  * geometries of any sizes, each with its own arguments -- with ONE CUDA graph
- * launch: cdfmm_b200_batch_create evaluates each plan once (building its
- * work tiles and tuning its M2L), then captures all the evaluations into one
+ * launch: cdfmm_b200_batch_create evaluates each plan once (building what a
+ * first call builds), then captures all the evaluations into one
  * graph whose per-geometry branches run concurrently.  Arguments are fixed at
  * creation and must be device-resident (memory == 0); a plan appears at most
  * once per batch and must not be evaluated by other calls while the batch is
@@ -355,8 +355,8 @@ int cdfmm_b200_batch_launch(cdfmm_b200_batch *batch, void *stream, int32_t synch
  * operators are the same), instead of one M2L per plan.  Writes each plan's
  * group (or -1: evaluated on its own) into out[capacity] and returns the
  * plan count.  A stacked plan's results may differ from its own evaluate at
- * FP32 rounding level (the group's M2L pipeline shape is chosen for the
- * group). */
+ * FP32 rounding level (the group's M2L splits its sums as the group's size
+ * asks). */
 int cdfmm_b200_batch_groups(const cdfmm_b200_batch *batch, int32_t *out, int32_t capacity);
 void cdfmm_b200_batch_destroy(cdfmm_b200_batch *batch);
 
@@ -380,8 +380,8 @@ int cdfmm_b200_set_timing(cdfmm_b200_plan *plan, int32_t enabled);
  * reference, which overlaps a cuSPARSE near field with its M2L on two
  * streams, src/cuda_fmm.cu:3295-3300, 3386-3391 upstream):
  * CDFMM_B200_SCHEDULE_*.  Both schedules compute the same sums; the near
- * field's summation order differs between them (state blocks of 64 vs 32)
- * and the M2L pipeline shape may too, at FP32 rounding level.  Evaluations
+ * field's summation order differs between them (state blocks of 64 vs 32),
+ * at FP32 rounding level.  Evaluations
  * whose M2L runs on the FP32 SIMT path always run SEPARATE. */
 int cdfmm_b200_set_schedule(cdfmm_b200_plan *plan, int32_t schedule);
 
@@ -408,13 +408,12 @@ int cdfmm_b200_get_stats(const cdfmm_b200_plan *plan, cdfmm_b200_stats *out);
  * CudaFull M2L has one fixed shape).  cdfmm_b200_m2l_shapes writes up to
  * `capacity` shapes as (accumulators per CTA, stages, fused) triples into
  * `out` ([capacity][3], may be NULL with capacity 0) and returns how many the
- * plan supports (negative: an error code).  By default the first
- * tensor-core evaluate of each K times them all and keeps the fastest; shapes
- * that differ only in accumulators or stages give bit-identical results,
- * the fused form (A_hi x [B_hi | B_lo] in one MMA) differs at FP32 rounding,
- * so timing noise can switch results at that level between runs.
- * cdfmm_b200_set_m2l_shape pins one of the listed shapes (no timing, the
- * same results on every run); m_tiles = 0 returns to autotuning. */
+ * plan supports (negative: an error code).  The first is the default, chosen
+ * from the order alone; how a tile's sum is split over CTAs follows from the
+ * tree, the order and K.  Shapes that differ only in stages give bit-identical
+ * results, the fused form (the hi x lo product in an accumulator of its own)
+ * differs at FP32 rounding.  cdfmm_b200_set_m2l_shape pins one of the listed
+ * shapes; m_tiles = 0 returns to the default. */
 int cdfmm_b200_m2l_shapes(const cdfmm_b200_plan *plan, int32_t *out, int32_t capacity);
 int cdfmm_b200_set_m2l_shape(cdfmm_b200_plan *plan, int32_t m_tiles, int32_t stages, int32_t fused);
 
