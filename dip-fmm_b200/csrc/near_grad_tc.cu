@@ -306,35 +306,40 @@ __global__ void __launch_bounds__(kNgThreads, 2) near_grad_tc_kernel(const NgArg
     // chunk i - 2; per k-step of 8 states three MMAs (A_hi B_hi, A_hi B_lo,
     // A_lo B_hi), N = 48.  B: core matrices 8 rows x 4 states, row groups
     // 128 bytes apart (SBO), state groups 768 bytes (LBO), lo after hi.
-    if (lane == 0) {
+    // The whole warp runs the loop and one lane issues (warp-uniform loop
+    // variables and descriptors; see near_tc.cu).
+    {
       const uint32_t idesc = instr_desc_tf32(kNgRows);
       const uint64_t desc0 = smem_desc(smem_u32(smem), kNgRows * 16u, 128u);
       const uint32_t lo_off = (static_cast<uint32_t>(Kpad) / 4u * kNgRows * 16u) >> 4;
-      bool ok = chunks == 0 || ng_wait(aready, 0, a.wait_limit);
-      if (!ok) ng_abort(abort_flag, a.error_flag, 9);
+      bool ok = __all_sync(0xffffffffu, chunks == 0 || ng_wait(aready, 0, a.wait_limit));
+      if (!ok && lane == 0) ng_abort(abort_flag, a.error_flag, 9);
       for (int i = 0; ok && i < chunks; ++i) {
         const int s = i % SB;
         const int db = i & 1;
-        if ((i >= 2 && !ng_wait(&dempty[db], static_cast<uint32_t>((i / 2) - 1) & 1u, a.wait_limit)) ||
-            !ng_wait(&bfull[s], static_cast<uint32_t>(i / SB) & 1u, a.wait_limit)) {
-          ng_abort(abort_flag, a.error_flag, 9);
+        bool go = i < 2 || ng_wait(&dempty[db], static_cast<uint32_t>((i / 2) - 1) & 1u, a.wait_limit);
+        go = go && ng_wait(&bfull[s], static_cast<uint32_t>(i / SB) & 1u, a.wait_limit);
+        if (!__all_sync(0xffffffffu, go)) {
+          if (lane == 0) ng_abort(abort_flag, a.error_flag, 9);
           break;
         }
         tc_fence_after();
-        const uint32_t dcol = tmem + dcol0 + static_cast<uint32_t>(db * kNgRows);
-        const uint64_t bd = desc0 + ((static_cast<uint32_t>(s) * lay.slot_bytes) >> 4);
-        for (int j = 0; j < Kpad / 8; ++j) {
-          const uint64_t bh = bd + ((2u * static_cast<uint32_t>(j) * kNgRows * 16u) >> 4);
-          const uint32_t ah = tmem + 8u * static_cast<uint32_t>(j);
-          const uint32_t al = ah + static_cast<uint32_t>(Kpad);
-          mma_tf32_ts(dcol, ah, bh, idesc, j == 0 ? 0u : 1u);
-          mma_tf32_ts(dcol, ah, bh + lo_off, idesc, 1);
-          mma_tf32_ts(dcol, al, bh, idesc, 1);
+        if (lane == 0) {
+          const uint32_t dcol = tmem + dcol0 + static_cast<uint32_t>(db * kNgRows);
+          const uint64_t bd = desc0 + ((static_cast<uint32_t>(s) * lay.slot_bytes) >> 4);
+          for (int j = 0; j < Kpad / 8; ++j) {
+            const uint64_t bh = bd + ((2u * static_cast<uint32_t>(j) * kNgRows * 16u) >> 4);
+            const uint32_t ah = tmem + 8u * static_cast<uint32_t>(j);
+            const uint32_t al = ah + static_cast<uint32_t>(Kpad);
+            mma_tf32_ts(dcol, ah, bh, idesc, j == 0 ? 0u : 1u);
+            mma_tf32_ts(dcol, ah, bh + lo_off, idesc, 1);
+            mma_tf32_ts(dcol, al, bh, idesc, 1);
+          }
+          mma_commit(&bempty[s]);
+          mma_commit(&dfull[db]);
         }
-        mma_commit(&bempty[s]);
-        mma_commit(&dfull[db]);
       }
-      mma_commit(done);
+      if (lane == 0) mma_commit(done);
     }
     __syncwarp();
   } else {

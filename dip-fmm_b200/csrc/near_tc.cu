@@ -397,49 +397,59 @@ __global__ void __launch_bounds__(kNtThreads, kNtCtasPerSm) near_tc_kernel(const
     // halves.  B descriptors: core matrices 8 states x 4 sources, the
     // 16 hi and lo state groups 128 bytes apart (SBO), K-adjacent core
     // matrices 32 N bytes apart (LBO).
-    if (lane == 0) {
+    // The whole warp runs the loop and one lane issues: loop variables,
+    // descriptors and slot counters are then warp-uniform.  (As one thread's
+    // loop, with divisions for the slots, the issue was the critical path:
+    // N = 131,072, K = 16 1.62 -> 1.44 ms, N = 1M, K = 64 14.5 -> 13.4 ms.)
+    {
       const uint32_t idesc = instr_desc_tf32(N);
       const uint32_t idesc2 = instr_desc_tf32(2 * N);
       const uint64_t desc0 = smem_desc(smem_u32(smem), 32u * static_cast<uint32_t>(N), 128u);
+      const uint64_t b_step = (64u * static_cast<uint32_t>(N)) >> 4, b_lo = (16u * static_cast<uint32_t>(N)) >> 4;
+      int sa = 0;           // A slot of chunk i and its phase
+      uint32_t pa = 0;
       for (int i = 0; i < chunks; ++i) {
         const int sb = i % SB;
-        const int sa = i % SA;
         const int gi = i / G;
         const int db = gi % kNtDBuf;
         const bool first = i % G == 0;
-        if (first && gi >= kNtDBuf &&
-            !nt_wait(&dfree[db], static_cast<uint32_t>((gi / kNtDBuf) - 1) & 1u, a.wait_limit)) {
-          nt_abort(abort_flag, a.error_flag, 5);
-          break;
-        }
-        if (!nt_wait(&bfull[sb], static_cast<uint32_t>(i / SB) & 1u, a.wait_limit) ||
-            !nt_wait(&aready[sa], static_cast<uint32_t>(i / SA) & 1u, a.wait_limit)) {
-          nt_abort(abort_flag, a.error_flag, 5);
+        bool ok = true;
+        if (first && gi >= kNtDBuf) ok = nt_wait(&dfree[db], static_cast<uint32_t>((gi / kNtDBuf) - 1) & 1u, a.wait_limit);
+        ok = ok && nt_wait(&bfull[sb], static_cast<uint32_t>(i / SB) & 1u, a.wait_limit) &&
+             nt_wait(&aready[sa], pa, a.wait_limit);
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (lane == 0) nt_abort(abort_flag, a.error_flag, 5);
           break;
         }
         tc_fence_after();
-        const uint32_t dcol = tmem + static_cast<uint32_t>(db) * acc_cols;
-        const uint64_t bd = desc0 + ((static_cast<uint32_t>(sb) * lay.slot_bytes) >> 4);
-        const uint32_t acol = tmem + acol0 + kNtAW * static_cast<uint32_t>(sa);
+        if (lane == 0) {
+          const uint32_t dcol = tmem + static_cast<uint32_t>(db) * acc_cols;
+          const uint64_t bd = desc0 + ((static_cast<uint32_t>(sb) * lay.slot_bytes) >> 4);
+          const uint32_t acol = tmem + acol0 + kNtAW * static_cast<uint32_t>(sa);
 #pragma unroll
-        for (int j = 0; j < 3 * kNtCB / 2; ++j) {
-          const uint64_t bj = bd + ((2u * static_cast<uint32_t>(j) * 32u * static_cast<uint32_t>(N)) >> 4);
-          const uint32_t ah = acol + 8u * static_cast<uint32_t>(j);
-          const uint32_t al = ah + 12u * kNtCB;
-          if (kNtFuse) {
-            mma_tf32_ts(dcol, ah, bj, idesc2, (first && j == 0) ? 0u : 1u);
-          } else {
-            mma_tf32_ts(dcol, ah, bj, idesc, (first && j == 0) ? 0u : 1u);
-            mma_tf32_ts(dcol, ah, bj + ((16u * static_cast<uint32_t>(N)) >> 4), idesc, 1); // B_lo
+          for (int j = 0; j < 3 * kNtCB / 2; ++j) {
+            const uint64_t bj = bd + static_cast<uint64_t>(j) * b_step;
+            const uint32_t ah = acol + 8u * static_cast<uint32_t>(j);
+            const uint32_t al = ah + 12u * kNtCB;
+            if (kNtFuse) {
+              mma_tf32_ts(dcol, ah, bj, idesc2, (first && j == 0) ? 0u : 1u);
+            } else {
+              mma_tf32_ts(dcol, ah, bj, idesc, (first && j == 0) ? 0u : 1u);
+              mma_tf32_ts(dcol, ah, bj + b_lo, idesc, 1);
+            }
+            mma_tf32_ts(dcol, al, bj, idesc, 1);
           }
-          mma_tf32_ts(dcol, al, bj, idesc, 1);
+          mma_commit(&bempty[sb]);
+          mma_commit(&aempty[sa]);
+          if (i % G == G - 1 || i == chunks - 1) mma_commit(&dready[db]);
         }
-        mma_commit(&bempty[sb]);
-        mma_commit(&aempty[sa]);
-        if (i % G == G - 1 || i == chunks - 1) mma_commit(&dready[db]);
+        if (++sa == SA) {
+          sa = 0;
+          pa ^= 1u;
+        }
       }
       // arrives once every MMA issued above has completed
-      mma_commit(done);
+      if (lane == 0) mma_commit(done);
     }
     __syncwarp();
   } else if (warp < 4 * kNtWg) {
@@ -472,10 +482,11 @@ __global__ void __launch_bounds__(kNtThreads, kNtCtasPerSm) near_tc_kernel(const
       agen_bar();
     }
     float4 *scratch = spos + 4 * (kNtPosCap + kNtCB) + 8 * warp; // this warp's 8 positions (unstaged)
+    int sa = wg % SA;            // A slot of chunk i, and the phase its previous use ends
+    uint32_t pa = 1u ^ (static_cast<uint32_t>(wg / SA) & 1u);
     for (int i = wg; ok && i < chunks; i += kNtWg) {
-      const int sa = i % SA;
       // the MMAs that read this slot's previous A (chunk i - SA) have completed
-      bool free_slot = i < SA || nt_wait(&aempty[sa], static_cast<uint32_t>((i / SA) - 1) & 1u, a.wait_limit);
+      bool free_slot = i < SA || nt_wait(&aempty[sa], pa, a.wait_limit);
       free_slot = __all_sync(0xffffffffu, free_slot);
       int go = free_slot ? 1 : 0;
       if (lane == 0) {
@@ -525,6 +536,7 @@ __global__ void __launch_bounds__(kNtThreads, kNtCtasPerSm) near_tc_kernel(const
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&aready[sa]);
+      for (sa += kNtWg; sa >= SA; sa -= SA) pa ^= 1u;
     }
   } else if (warp >= kNtDrainWarp) {
     // Drains: warp kNtDrainWarp + r reads the rows of tensor-memory
