@@ -361,40 +361,36 @@ __global__ void __launch_bounds__(kTcThreads, 1) m2l_tc_kernel(const __grid_cons
   }
 }
 
-// Sum of the splits' reduced locals into the first split's, in a fixed order:
-// a CTA takes 32 float4 positions, its 8 groups of threads every eighth split
-// (the splits of one position are all the loads there are when the tree is
-// small).
-constexpr int kSumItems = 32, kSumGroups = 8;
+// Sum of the splits' reduced locals into the first split's, in a fixed order.
+// Many splits (16 and more: small trees, where they are all the loads there
+// are) are taken by 8 groups of threads, group g every eighth split; few by one
+// thread per position (N = 1M, p = 6, K = 1, 3 splits: 8 groups took 31 us).
+constexpr int kSumThreads = 256, kSumGroups = 8;
 
-__global__ void __launch_bounds__(kSumItems * kSumGroups) m2l_sum_splits_kernel(float4 *__restrict__ R, long long vec,
-                                                                                int splits) {
-  __shared__ float4 part[kSumGroups][kSumItems];
-  const int item = threadIdx.x % kSumItems, group = threadIdx.x / kSumItems;
-  const long long at = static_cast<long long>(blockIdx.x) * kSumItems + item;
+template <int GROUPS>
+__global__ void __launch_bounds__(kSumThreads) m2l_sum_splits_kernel(float4 *__restrict__ R, long long vec, int splits) {
+  constexpr int items = kSumThreads / GROUPS;
+  __shared__ float4 part[kSumThreads];
+  const int item = threadIdx.x % items, group = threadIdx.x / items;
+  const long long at = static_cast<long long>(blockIdx.x) * items + item;
   float4 v = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+  auto add = [&v](const float4 &x) {
+    v.x += x.x;
+    v.y += x.y;
+    v.z += x.z;
+    v.w += x.w;
+  };
   if (at < vec) {
 #pragma unroll 4
-    for (int s = group; s < splits; s += kSumGroups) {
-      const float4 x = R[at + s * vec];
-      v.x += x.x;
-      v.y += x.y;
-      v.z += x.z;
-      v.w += x.w;
-    }
+    for (int s = group; s < splits; s += GROUPS) add(R[at + s * vec]);
   }
-  part[group][item] = v;
-  __syncthreads();
-  if (group == 0 && at < vec) {
-    for (int g = 1; g < kSumGroups; ++g) {
-      const float4 x = part[g][item];
-      v.x += x.x;
-      v.y += x.y;
-      v.z += x.z;
-      v.w += x.w;
-    }
-    R[at] = v;
+  if constexpr (GROUPS > 1) {
+    part[threadIdx.x] = v;
+    __syncthreads();
+    if (group == 0)
+      for (int g = 1; g < GROUPS; ++g) add(part[g * items + item]);
   }
+  if (group == 0 && at < vec) R[at] = v;
 }
 
 // Pack: multipoles of levels 2..depth, folded, scaled and split into BF16
@@ -741,8 +737,12 @@ int launch_m2l_tc(const M2lTcArgs &args, cudaStream_t s) {
   m2l_tc_kernel<<<args.tiles * args.groups * args.splits, kTcThreads, smem, s>>>(args);
   if (args.splits == 1) return 1;
   const long long vec = args.split_stride / 4; // a multiple of 64 boxes
-  m2l_sum_splits_kernel<<<static_cast<unsigned>((vec + kSumItems - 1) / kSumItems), kSumItems * kSumGroups, 0, s>>>(
-      reinterpret_cast<float4 *>(args.R), vec, args.splits);
+  float4 *R = reinterpret_cast<float4 *>(args.R);
+  const auto grid = [vec](int items) { return static_cast<unsigned>((vec + items - 1) / items); };
+  if (args.splits >= 16)
+    m2l_sum_splits_kernel<kSumGroups><<<grid(kSumThreads / kSumGroups), kSumThreads, 0, s>>>(R, vec, args.splits);
+  else
+    m2l_sum_splits_kernel<1><<<grid(kSumThreads), kSumThreads, 0, s>>>(R, vec, args.splits);
   return 2;
 }
 
