@@ -193,8 +193,8 @@ struct cdfmm_b200_plan {
   int *ntc_blk_off = nullptr;
   int *ntc_blk_src = nullptr;
   float4 *ntc_blk_pos = nullptr;
-  int4 *ntc_work = nullptr;
-  int ntc_n_blocks = 0, ntc_n_work = 0;
+  int4 *ntc_work = nullptr, *ntc_work_field = nullptr;
+  int ntc_n_blocks = 0, ntc_n_work = 0, ntc_n_work_field = 0;
   void *ntc_b = nullptr;
   // tensor-core position gradient of the near field: blocks of 16 sources
   bool ngt_supported = false;

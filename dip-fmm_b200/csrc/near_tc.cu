@@ -83,7 +83,7 @@ constexpr int kNtMmaWarp = kNtCopyWarp + 1;
 constexpr int kNtDrainWarp = kNtCopyWarp + 2; // four drain warps
 constexpr int kNtThreads = 32 * (kNtDrainWarp + 4);
 constexpr uint32_t kNtTmemCols = kNtCtasPerSm == 2 ? 256 : 512;
-constexpr int kNtStageStride = 33;    // epilogue transpose row (32 targets + 1)
+constexpr int kNtStageStride = 129;   // epilogue transpose row (128 rows + 1)
 constexpr int kNtPosCap = 384;        // neighbourhood blocks whose positions are staged in shared memory
 // Blocks of 4 sources per pipeline chunk (even), and whether a k-step's
 // hi x hi and hi x lo products run as one MMA of width 2 K (A_hi x
@@ -109,7 +109,8 @@ constexpr uint32_t kNtMiscBytes = 640;
 #endif
 
 // Accumulator buffers: 2 (the MMAs of the next group run while a group is
-// drained) or 1 (more A slots; the MMAs wait for each drain).
+// drained; no faster even where both fit beside two A slots, K <= 32) or 1
+// (the MMAs wait for each drain).
 #ifndef CDFMM_NTC_DBUF
 #define CDFMM_NTC_DBUF 1
 #endif
@@ -127,7 +128,7 @@ __host__ __device__ inline int nt_slots(int N) {
 struct NtSmem {
   uint32_t slot_bytes; // 2 blocks of [3 components][hi, lo][N states][4 sources]
   uint32_t pos_off;    // staged neighbourhood positions [kNtPosCap + 1][4] float4, then [4 kNtWg][8] scratch
-  uint32_t stage_off;  // epilogue transpose [4 components][16 states][33]
+  uint32_t stage_off;  // epilogue transpose [16 states][129]
   uint32_t bar_off;
   uint32_t misc_off;
   uint32_t total;
@@ -137,7 +138,7 @@ __host__ __device__ inline NtSmem nt_smem(int N, int SA) {
   m.slot_bytes = 96u * kNtCB * static_cast<uint32_t>(N);
   m.pos_off = kNtBSlots * m.slot_bytes;
   m.stage_off = m.pos_off + (kNtPosCap + kNtCB) * 64u + 4u * kNtWg * 128u;
-  m.bar_off = m.stage_off + 4u * 16u * kNtStageStride * 4u;
+  m.bar_off = (m.stage_off + 16u * kNtStageStride * 4u + 7u) & ~7u;
   m.misc_off = m.bar_off + (2u * kNtBSlots + 2u * static_cast<uint32_t>(SA) + 6u) * 8u;
   m.total = m.misc_off + kNtMiscBytes;
   return m;
@@ -152,7 +153,7 @@ struct NtArgs {
   const int *self_idx;
   float4 *near;
   int *error_flag;
-  int depth, K, N, slots, want_phi, zero_block;
+  int depth, K, N, slots, zero_block;
   uint32_t wait_limit;
 };
 
@@ -216,6 +217,42 @@ __device__ __forceinline__ void chunk_tensors(const float4 *p8, float ntx, float
   }
 }
 
+// The tensors of one field component chosen per lane (0, 1, 2 = x, y, z; `on`
+// holds 1 at that component, else 0), bit for bit those of chunk_tensors.
+__device__ __forceinline__ void chunk_tensors_field(const float4 *p8, float ntx, float nty, float ntz, int self,
+                                                    int comp, const float (&on)[3], float *hv, float *lv) {
+#pragma unroll
+  for (int pr = 0; pr < 4; ++pr) {
+    const float4 p0 = p8[2 * pr], p1 = p8[2 * pr + 1];
+    const float2 dx = __fadd2_rn(make_float2(p0.x, p1.x), make_float2(ntx, ntx));
+    const float2 dy = __fadd2_rn(make_float2(p0.y, p1.y), make_float2(nty, nty));
+    const float2 dz = __fadd2_rn(make_float2(p0.z, p1.z), make_float2(ntz, ntz));
+    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+    float2 rinv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+    rinv.x = __float_as_int(p0.w) == self ? 0.0F : rinv.x;
+    rinv.y = __float_as_int(p1.w) == self ? 0.0F : rinv.y;
+    const float2 rinv2 = __fmul2_rn(rinv, rinv);
+    const float2 v = __fmul2_rn(rinv2, rinv);
+    const float2 nv = __fmul2_rn(v, make_float2(-1.0F, -1.0F));
+    const float2 f = __fmul2_rn(__fmul2_rn(v, rinv2), make_float2(3.0F, 3.0F));
+    const float2 dc = make_float2(comp == 0 ? dx.x : comp == 1 ? dy.x : dz.x, comp == 0 ? dx.y : comp == 1 ? dy.y : dz.y);
+    const float2 g = __fmul2_rn(f, dc);
+    const float2 e[3] = {__ffma2_rn(g, dx, __fmul2_rn(nv, make_float2(on[0], on[0]))),
+                         __ffma2_rn(g, dy, __fmul2_rn(nv, make_float2(on[1], on[1]))),
+                         __ffma2_rn(g, dz, __fmul2_rn(nv, make_float2(on[2], on[2])))};
+    const int col = 12 * (pr >> 1) + 2 * (pr & 1);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      float2 hi, lo;
+      split_tf32x2(e[d], hi, lo);
+      hv[col + 4 * d] = hi.x;
+      hv[col + 4 * d + 1] = hi.y;
+      lv[col + 4 * d] = lo.x;
+      lv[col + 4 * d + 1] = lo.y;
+    }
+  }
+}
+
 __device__ __forceinline__ float4 far_slot() {
   return make_float4(3.0e18F, 3.0e18F, 3.0e18F, __int_as_float(-1));
 }
@@ -245,6 +282,10 @@ __device__ __forceinline__ bool nt_aborted(const int *abort_flag) {
   return *reinterpret_cast<const volatile int *>(abort_flag) != 0;
 }
 
+// FIELD: no potential, so the 128 rows are 3 components x 42 targets (row 42
+// c + t; two rows idle) instead of 4 x 32.  A leaf of about 32 then is one unit
+// where it was 1.46 on average, and each chunk's fixed work serves 42 targets.
+template <bool FIELD>
 __global__ void __launch_bounds__(kNtThreads, kNtCtasPerSm) near_tc_kernel(const NtArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x;
@@ -457,10 +498,13 @@ __global__ void __launch_bounds__(kNtThreads, kNtCtasPerSm) near_tc_kernel(const
     // warp c forms the row block of component c, lane t target t.
     const int c = warp & 3;
     const int wg = warp >> 2;
-    const int it = t0 + (lane < nt ? lane : 0); // lanes beyond the unit's targets: rows never stored
+    const int comp = FIELD ? min((32 * c + lane) / kNearTcFieldTargets, 2) : 0;
+    const int tl = FIELD ? 32 * c + lane - kNearTcFieldTargets * comp : lane; // this row's target
+    const float on[3] = {comp == 0 ? 1.0F : 0.0F, comp == 1 ? 1.0F : 0.0F, comp == 2 ? 1.0F : 0.0F};
+    const int it = t0 + (tl < nt ? tl : 0); // rows beyond the unit's targets: never stored
     const float4 tp = a.tgt_rel[it];
     const float ntx = -tp.x, nty = -tp.y, ntz = -tp.z;
-    const int self = (a.self_idx != nullptr && lane < nt) ? a.self_idx[it] : -2;
+    const int self = (a.self_idx != nullptr && tl < nt) ? a.self_idx[it] : -2;
     const uint32_t lane_base = static_cast<uint32_t>(32 * c) << 16;
     bool ok = true;
     if (staged && chunks > 0) ok = nt_wait(pfull, 0, a.wait_limit);
@@ -519,11 +563,15 @@ __global__ void __launch_bounds__(kNtThreads, kNtCtasPerSm) near_tc_kernel(const
           p8 = scratch;
         }
         float hv[24], lv[24];
-        switch (c) {
-        case 0: chunk_tensors<0>(p8, ntx, nty, ntz, self, hv, lv); break;
-        case 1: chunk_tensors<1>(p8, ntx, nty, ntz, self, hv, lv); break;
-        case 2: chunk_tensors<2>(p8, ntx, nty, ntz, self, hv, lv); break;
-        default: chunk_tensors<3>(p8, ntx, nty, ntz, self, hv, lv); break;
+        if constexpr (FIELD) {
+          chunk_tensors_field(p8, ntx, nty, ntz, self, comp, on, hv, lv);
+        } else {
+          switch (c) {
+          case 0: chunk_tensors<0>(p8, ntx, nty, ntz, self, hv, lv); break;
+          case 1: chunk_tensors<1>(p8, ntx, nty, ntz, self, hv, lv); break;
+          case 2: chunk_tensors<2>(p8, ntx, nty, ntz, self, hv, lv); break;
+          default: chunk_tensors<3>(p8, ntx, nty, ntz, self, hv, lv); break;
+          }
         }
         if (!staged) __syncwarp(); // scratch reads done before the next sub-chunk overwrites it
         const uint32_t th = ta + 24u * static_cast<uint32_t>(h);
@@ -588,23 +636,23 @@ __global__ void __launch_bounds__(kNtThreads, kNtCtasPerSm) near_tc_kernel(const
       poison = poison || nt_aborted(abort_flag);
     }
     poison = __shfl_sync(0xffffffffu, poison, 0);
-    const float scale = (c == 0 && !a.want_phi) ? 0.0F : kInvFourPiF;
     const int et = tid - 32 * kNtDrainWarp; // 0..127 over the drain warps
+    constexpr int T = FIELD ? kNearTcFieldTargets : kNearTcTargets; // rows T per component
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (16 * q < N) {
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
-          stage[(c * 16 + kk) * kNtStageStride + lane] = poison ? __int_as_float(0x7fc00000) : acc[q][kk] * scale;
+          stage[kk * kNtStageStride + 32 * c + lane] = poison ? __int_as_float(0x7fc00000) : acc[q][kk] * kInvFourPiF;
         drain_bar();
-        for (int e = et; e < 32 * 16; e += 128) {
+        for (int e = et; e < T * 16; e += 128) {
           const int tt = e >> 4;
           const int kk = e & 15;
           const int k = 16 * q + kk;
+          const float *row = stage + kk * kNtStageStride + tt;
           if (tt < nt && k < a.K)
             a.near[static_cast<long long>(t0 + tt) * a.K + k] =
-                make_float4(stage[kk * kNtStageStride + tt], stage[(16 + kk) * kNtStageStride + tt],
-                            stage[(32 + kk) * kNtStageStride + tt], stage[(48 + kk) * kNtStageStride + tt]);
+                FIELD ? make_float4(0.0F, row[0], row[T], row[2 * T]) : make_float4(row[0], row[T], row[2 * T], row[3 * T]);
         }
         drain_bar();
       }
@@ -726,6 +774,8 @@ NearTcLayout near_tc_layout(const int *src_off, const int *tgt_off, int depth) {
       lay.work.push_back(make_int4(l, tgt_off[l] + t, std::min(kNearTcTargets, tn - t), cost));
       lay.k_cols += 3u * 4u * static_cast<uint64_t>(kNtCB) * static_cast<uint64_t>((cost + kNtCB - 1) / kNtCB);
     }
+    for (int t = 0; t < tn; t += kNearTcFieldTargets)
+      lay.work_field.push_back(make_int4(l, tgt_off[l] + t, std::min(kNearTcFieldTargets, tn - t), cost));
   }
   return lay;
 }
@@ -757,7 +807,12 @@ void launch_near_tc(const NearTcLaunch &a, const float4 *mom, const float4 *tgt_
   args.blk_pos = a.blk_pos;
   args.blk_off = a.blk_off;
   args.b_ops = static_cast<const uint8_t *>(a.b_ops);
-  args.work = a.work;
+  // Without the potential the 42-target form, where it has at least a tenth
+  // fewer units (its per-lane components cost about that; 8 targets per leaf,
+  // p = 8 lattice, K = 64: 3.1 against 2.8 ms with as many units either way;
+  // 32 per leaf, N = 131,072, K = 16: 1.23 against 1.44 ms with 0.72 of them).
+  const bool field = !want_phi && 10LL * a.n_work_field <= 9LL * a.n_work;
+  args.work = field ? a.work_field : a.work;
   args.tgt_rel = tgt_rel;
   args.self_idx = self_idx;
   args.near = near;
@@ -766,18 +821,21 @@ void launch_near_tc(const NearTcLaunch &a, const float4 *mom, const float4 *tgt_
   args.K = K;
   args.N = N;
   args.slots = nt_slots(N);
-  args.want_phi = want_phi ? 1 : 0;
   args.zero_block = a.n_blocks;
   args.wait_limit = a.wait_limit;
   // Enough shared memory per CTA that no more CTAs than the tensor memory
   // holds share an SM (the extra one's allocation would wait for ours).
   const size_t smem = std::max<size_t>(nt_smem(N, args.slots).total, kNtCtasPerSm == 2 ? 80 * 1024 : 116 * 1024);
-  near_tc_kernel<<<a.n_work, kNtThreads, smem, s>>>(args);
+  if (field)
+    near_tc_kernel<true><<<a.n_work_field, kNtThreads, smem, s>>>(args);
+  else
+    near_tc_kernel<false><<<a.n_work, kNtThreads, smem, s>>>(args);
 }
 
 bool configure_near_tc(size_t max_smem) {
-  prefer_max_shared_carveout(near_tc_kernel);
-  return allow_dynamic_smem(near_tc_kernel, max_smem);
+  prefer_max_shared_carveout(near_tc_kernel<false>);
+  prefer_max_shared_carveout(near_tc_kernel<true>);
+  return allow_dynamic_smem(near_tc_kernel<false>, max_smem) && allow_dynamic_smem(near_tc_kernel<true>, max_smem);
 }
 
 } // namespace cdfmm_b200

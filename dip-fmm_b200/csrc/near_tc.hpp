@@ -14,6 +14,7 @@ namespace cdfmm_b200 {
 // padded with empty slots); a block is the unit of the moment operand.
 constexpr int kNearTcSlots = 4;      // sources per block
 constexpr int kNearTcTargets = 32;   // targets per work unit (128 rows = 4 components x 32)
+constexpr int kNearTcFieldTargets = 42; // without the potential (126 rows = 3 components x 42)
 constexpr int kNearTcMinStates = 8;  // K range served (MMA N = K rounded up to 16, <= 64)
 constexpr int kNearTcMaxStates = 64;
 
@@ -23,6 +24,7 @@ struct NearTcLayout {
   std::vector<int> blk_off; // [leaves + 1] first block of each leaf
   std::vector<int> blk_src; // [(n_blocks + 1) * 4] sorted source index of each slot, -1: empty
   std::vector<int4> work;   // (leaf, first target, targets <= 32, neighbourhood blocks) in leaf order
+  std::vector<int4> work_field; // the same with targets <= 42 (no potential)
   int n_blocks = 0;         // block n_blocks is the all-empty block
   uint64_t k_cols = 0;      // sum over units of the MMA reduction length (3 x chunk-padded sources)
 };
@@ -36,6 +38,8 @@ struct NearTcLaunch {
   int n_blocks;
   const int4 *work;
   int n_work;
+  const int4 *work_field; // units of the evaluations without the potential
+  int n_work_field;
   void *b_ops;           // [(n_blocks + 1)][3][hi, lo][N][4] TF32 moments (96 N bytes per block)
   int *error_flag;
   uint32_t wait_limit;

@@ -116,7 +116,7 @@ void free_plan(cdfmm_b200_plan *p) {
                   p->tc_R, p->m2l_fold_buf, p->tc_fold_off, p->tc_fold, p->tc_expand, p->error_flag, p->wbuf, p->gpart, p->stage_grad, p->p2p_next_unit,
                   p->close_targets, p->close_r_fp32, p->close_r_exact, p->src_pos64, p->tgt_pos64,
                   p->src_size, p->src_size64, p->cuboid_T, p->cuboid_base, p->ntc_blk_off, p->ntc_blk_src,
-                  p->ntc_blk_pos, p->ntc_work, p->ntc_b, p->ngt_blk_off, p->ngt_blk_src, p->ngt_blk_pos,
+                  p->ntc_blk_pos, p->ntc_work, p->ntc_work_field, p->ntc_b, p->ngt_blk_off, p->ngt_blk_src, p->ngt_blk_pos,
                   p->ngt_b};
   for (void *q : ptrs)
     if (q != nullptr) cudaFree(q);
@@ -1077,6 +1077,8 @@ static void ensure_near_tc(cdfmm_b200_plan *plan) {
   plan->ntc_blk_pos = dalloc<float4>(lay.blk_src.size(), bytes);
   plan->ntc_work = dalloc<int4>(lay.work.size(), bytes);
   upload(plan->ntc_work, lay.work.data(), lay.work.size(), h2d);
+  plan->ntc_work_field = dalloc<int4>(lay.work_field.size(), bytes);
+  upload(plan->ntc_work_field, lay.work_field.data(), lay.work_field.size(), h2d);
   const size_t ob = near_tc_operand_bytes(lay.n_blocks, std::min(plan->max_states, kNearTcMaxStates));
   plan->ntc_b = dalloc<uint8_t>(ob, bytes);
   launch_near_tc_positions(plan->src_rel, plan->ntc_blk_src, lay.n_blocks, plan->ntc_blk_pos, plan->stream);
@@ -1084,6 +1086,7 @@ static void ensure_near_tc(cdfmm_b200_plan *plan) {
   check(cudaStreamSynchronize(plan->stream), "near-field blocks");
   plan->ntc_n_blocks = lay.n_blocks;
   plan->ntc_n_work = static_cast<int>(lay.work.size());
+  plan->ntc_n_work_field = static_cast<int>(lay.work_field.size());
   plan->stats.near_tc_k_cols = lay.k_cols;
   plan->stats.persistent_device_bytes += bytes;
   plan->stats.setup_h2d_bytes += h2d;
@@ -1121,6 +1124,8 @@ static NearTcLaunch near_tc_launch(const cdfmm_b200_plan *plan) {
   l.n_blocks = plan->ntc_n_blocks;
   l.work = plan->ntc_work;
   l.n_work = plan->ntc_n_work;
+  l.work_field = plan->ntc_work_field;
+  l.n_work_field = plan->ntc_n_work_field;
   l.b_ops = plan->ntc_b;
   l.error_flag = plan->error_flag;
   l.wait_limit = plan->tc_wait_limit;
