@@ -433,27 +433,40 @@ __global__ void __launch_bounds__(kPackThreads) m2l_pack_kernel(const float *__r
       const int k = e / (8 * n), r = e - k * 8 * n;
       const int c = r / n, a = r - c * n;
       for (int q = 0; q < nP; ++q)
-        sM[a * kPackPitch + (q * kc + k) * 8 + c] = M_list[k0 + k][(child0 + 8 * q) * n + r];
+        cp_async4(sM + a * kPackPitch + (q * kc + k) * 8 + c, M_list[k0 + k] + (child0 + 8 * q) * n + r);
     }
   } else if ((K & 3) == 0) {
-    const int quads = kc >> 2;
-    for (int e = tid; e < nP * 8 * n * quads; e += kPackThreads) {
-      const int kq = e % quads, t = e / quads;
-      const int a = t % n, b = t / n; // box b of the CTA
-      const float4 v = *reinterpret_cast<const float4 *>(M + ((child0 + b) * n + a) * K + k0 + 4 * kq);
-      float *dst = sM + a * kPackPitch + ((b >> 3) * kc + 4 * kq) * 8 + (b & 7);
-      dst[0] = v.x;
-      dst[8] = v.y;
-      dst[16] = v.z;
-      dst[24] = v.w;
+    // (four loads in flight per thread)
+    const int quads = kc >> 2, total = nP * 8 * n * quads;
+    for (int e0 = tid; e0 < total; e0 += 4 * kPackThreads) {
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = e0 + i * kPackThreads, t = e / quads;
+        if (e < total)
+          v[i] = *reinterpret_cast<const float4 *>(M + (child0 * n + t) * K + k0 + 4 * (e - t * quads));
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = e0 + i * kPackThreads;
+        if (e >= total) break;
+        const int t = e / quads, kq = e - t * quads;
+        const int b = t / n, a = t - b * n; // box b of the CTA, coefficient a
+        float *dst = sM + a * kPackPitch + ((b >> 3) * kc + 4 * kq) * 8 + (b & 7);
+        dst[0] = v[i].x;
+        dst[8] = v[i].y;
+        dst[16] = v[i].z;
+        dst[24] = v[i].w;
+      }
     }
   } else {
     for (int e = tid; e < nP * 8 * n * kc; e += kPackThreads) {
       const int k = e % kc, t = e / kc;
       const int a = t % n, b = t / n;
-      sM[a * kPackPitch + ((b >> 3) * kc + k) * 8 + (b & 7)] = M[((child0 + b) * n + a) * K + k0 + k];
+      cp_async4(sM + a * kPackPitch + ((b >> 3) * kc + k) * 8 + (b & 7), M + ((child0 + b) * n + a) * K + k0 + k);
     }
   }
+  cp_async_commit();
   for (int e = tid; e <= n_in; e += kPackThreads) off[e] = __ldg(fold_off + e);
   for (int e = tid; e < n_fold; e += kPackThreads) {
     // the entries of one input are of one degree: its scaling 2^(level degree) is exact
@@ -464,6 +477,7 @@ __global__ void __launch_bounds__(kPackThreads) m2l_pack_kernel(const float *__r
     from[e] = a * kPackPitch;
     coef[e] = static_cast<float>((ent >> 16) - 64) * __int_as_float((127 + level * deg) << 23);
   }
+  cp_async_wait<0>();
   __syncthreads();
   // pairs of inputs: two folded moments, their hi and lo halves as one word each
   for (int e = tid; e < chunks * 8 * kPackCols; e += kPackThreads) {
