@@ -222,6 +222,9 @@ void UniformFmm::bind_identities(std::span<const int> ids, std::size_t moment_co
     identities_bound_ = true;
     return;
   }
+  // the plan's default map (the fixed one, or none) is bound already
+  const bool by_default = ids.empty();
+  if (by_default && identities_bound_ && default_bound_) return;
   const std::size_t nt = tree_.sorted_target_positions().size();
   if (fixed_identities_.has_value()) {
     const std::vector<int> &fixed = fixed_identities_.value();
@@ -248,7 +251,9 @@ void UniformFmm::bind_identities(std::span<const int> ids, std::size_t moment_co
       if (s >= 0) sorted[t] = sinv[static_cast<std::size_t>(s)];
     }
   }
+  default_bound_ = by_default;
   if (identities_bound_ && sorted == fixed_sorted_self_) return;
+  identities_bound_ = false; // (stays so if the upload fails)
   check_plan(cdfmm_b200_set_self_indices(plan_.get(), sorted.data()), plan_.get());
   fixed_sorted_self_ = std::move(sorted);
   identities_bound_ = true;

@@ -204,6 +204,7 @@ private:
   std::optional<std::vector<int>> fixed_identities_{};
   std::vector<int> fixed_sorted_self_{};
   bool identities_bound_{false};
+  bool default_bound_{false}; // the bound map is the one an evaluate without indices uses
   bool cuboid_sources_{false}; // identity maps do not apply to cuboid sources
   StaticPlanStatistics static_stats_{};
   mutable CudaPlanStatistics cuda_stats_{};
