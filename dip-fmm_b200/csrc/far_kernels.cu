@@ -15,6 +15,22 @@ namespace cdfmm_b200 {
 
 namespace {
 
+// Calls f(nu, kn) for a tile of nu points and kn states, both <= 32: as
+// compile-time constants for the full tiles (32 points, 32 or 16 states),
+// whose index arithmetic is then shifts and whose loops unroll.  (With
+// divisions at run time they ran at half of HBM.  N = 1,048,576, K = 64:
+// gather 607 -> 498 us, L2P and unsort 1793 -> 1660 us;
+// tiles of 8 states measured the same either way.)
+template <class F> __device__ __forceinline__ void with_tile(int nu, int kn, F f) {
+  using std::integral_constant;
+  if (nu == 32 && kn == 32)
+    f(integral_constant<int, 32>{}, integral_constant<int, 32>{});
+  else if (nu == 32 && kn == 16)
+    f(integral_constant<int, 32>{}, integral_constant<int, 16>{});
+  else
+    f(nu, kn);
+}
+
 // ---------------------------------------------------------------------------
 // moments: user order [K][ns][3] (f32 / f64) -> sorted [ns][K] float4 / scale^3
 // (upstream src/far_field.cpp:248-275, src/cuda_fmm.cu:56-64).  A CTA takes
@@ -28,46 +44,47 @@ __global__ void __launch_bounds__(256) gather_moments_kernel(const T *__restrict
                                                              int krow) {
   __shared__ float tile[32][32 * 3 + 1]; // [user][state * 3 + component]
   const int u0 = blockIdx.x * 32;
-  const int nu = min(32, ns - u0);
-  for (int kc = 0; kc < K; kc += 32) {
-    const int kn = min(32, K - kc);
-    for (int e = threadIdx.x; e < kn * nu * 3; e += blockDim.x) {
-      const int k = e / (nu * 3);
-      const int r = e - k * nu * 3;
-      const int t = r / 3;
-      const T v = user[(static_cast<long long>(kc + k) * ns + u0) * 3 + r];
-      float f;
-      if constexpr (sizeof(T) == 8)
-        f = static_cast<float>(static_cast<double>(v) * inv_scale * inv_scale * inv_scale); // m / s / s / s in FP64
-      else
-        f = static_cast<float>(v) * inv_scale3_f;
-      tile[t][3 * k + (r - 3 * t)] = f;
-    }
-    __syncthreads();
-    if (paired) {
-      // state pairs (k, k+1) as (x_k, x_k1, y_k, y_k1), (z_k, z_k1, 0, 0); a
-      // missing partner (K odd) is zero
-      const int kp = (kn + 1) >> 1;
-      const int row = krow;
-      for (int e = threadIdx.x; e < nu * kp; e += blockDim.x) {
-        const int t = e / kp;
-        const int k = 2 * (e - t * kp);
-        const bool b = k + 1 < kn;
-        float4 *dst = mom + static_cast<long long>(inv[u0 + t]) * row + k0 + kc + k;
-        dst[0] = make_float4(tile[t][3 * k], b ? tile[t][3 * k + 3] : 0.0F, tile[t][3 * k + 1],
-                             b ? tile[t][3 * k + 4] : 0.0F);
-        dst[1] = make_float4(tile[t][3 * k + 2], b ? tile[t][3 * k + 5] : 0.0F, 0.0F, 0.0F);
+  for (int kc = 0; kc < K; kc += 32)
+    with_tile(min(32, ns - u0), min(32, K - kc), [&](auto nu, auto kn) {
+#pragma unroll 4
+      for (int e = threadIdx.x; e < kn * nu * 3; e += 256) {
+        const int k = e / (nu * 3);
+        const int r = e - k * (nu * 3);
+        const int t = r / 3;
+        const T v = user[(static_cast<long long>(kc + k) * ns + u0) * 3 + r];
+        float f;
+        if constexpr (sizeof(T) == 8)
+          f = static_cast<float>(static_cast<double>(v) * inv_scale * inv_scale * inv_scale); // m / s / s / s in FP64
+        else
+          f = static_cast<float>(v) * inv_scale3_f;
+        tile[t][3 * k + (r - 3 * t)] = f;
       }
-    } else {
-      for (int e = threadIdx.x; e < nu * kn; e += blockDim.x) {
-        const int t = e / kn;
-        const int k = e - t * kn;
-        mom[static_cast<long long>(inv[u0 + t]) * krow + k0 + kc + k] =
-            make_float4(tile[t][3 * k], tile[t][3 * k + 1], tile[t][3 * k + 2], 0.0F);
+      __syncthreads();
+      if (paired) {
+        // state pairs (k, k+1) as (x_k, x_k1, y_k, y_k1), (z_k, z_k1, 0, 0); a
+        // missing partner (K odd) is zero
+        const int row = krow;
+#pragma unroll 2
+        for (int e = threadIdx.x; e < nu * ((kn + 1) / 2); e += 256) {
+          const int t = e / ((kn + 1) / 2);
+          const int k = 2 * (e - t * ((kn + 1) / 2));
+          const bool b = k + 1 < kn;
+          float4 *dst = mom + static_cast<long long>(inv[u0 + t]) * row + k0 + kc + k;
+          dst[0] = make_float4(tile[t][3 * k], b ? tile[t][3 * k + 3] : 0.0F, tile[t][3 * k + 1],
+                               b ? tile[t][3 * k + 4] : 0.0F);
+          dst[1] = make_float4(tile[t][3 * k + 2], b ? tile[t][3 * k + 5] : 0.0F, 0.0F, 0.0F);
+        }
+      } else {
+#pragma unroll 2
+        for (int e = threadIdx.x; e < nu * kn; e += 256) {
+          const int t = e / kn;
+          const int k = e - t * kn;
+          mom[static_cast<long long>(inv[u0 + t]) * krow + k0 + kc + k] =
+              make_float4(tile[t][3 * k], tile[t][3 * k + 1], tile[t][3 * k + 2], 0.0F);
+        }
       }
-    }
-    __syncthreads();
-  }
+      __syncthreads();
+    });
 }
 
 // Sorted results res[nt][K] (phi, Hx, Hy, Hz) -> user order: field[K][nt][3]
@@ -81,44 +98,47 @@ __global__ void __launch_bounds__(256) unsort_results_kernel(const float4 *__res
                                                              int k_begin, int k_end) {
   __shared__ float4 tile[32][33];
   const int u0 = blockIdx.x * 32;
-  const int nu = min(32, nt - u0);
   const bool want_phi = (output & 1u) != 0u;
   const bool want_h = (output & 2u) != 0u;
-  for (int kc = k_begin; kc < k_end; kc += 32) {
-    const int kn = min(32, k_end - kc);
-    for (int e = threadIdx.x; e < nu * kn; e += blockDim.x) {
-      const int t = e / kn;
-      const int k = e - t * kn;
-      tile[t][k] = res[static_cast<long long>(inv[u0 + t]) * K + kc + k];
-    }
-    __syncthreads();
-    if (layout == 1) {
-      for (int e = threadIdx.x; e < kn * nu; e += blockDim.x) {
-        const int k = e / nu;
-        const int t = e - k * nu;
-        reinterpret_cast<float4 *>(field)[static_cast<long long>(kc + k) * nt + u0 + t] = tile[t][k];
+  for (int kc = k_begin; kc < k_end; kc += 32)
+    with_tile(min(32, nt - u0), min(32, k_end - kc), [&](auto nu, auto kn) {
+#pragma unroll 4
+      for (int e = threadIdx.x; e < nu * kn; e += 256) {
+        const int t = e / kn;
+        const int k = e - t * kn;
+        tile[t][k] = res[static_cast<long long>(inv[u0 + t]) * K + kc + k];
       }
-    } else {
-      if (want_h) {
-        for (int e = threadIdx.x; e < kn * nu * 3; e += blockDim.x) {
-          const int k = e / (nu * 3);
-          const int r = e - k * nu * 3;
-          const int t = r / 3;
-          const int c = r - 3 * t;
-          const float4 v = tile[t][k];
-          field[(static_cast<long long>(kc + k) * nt + u0) * 3 + r] = c == 0 ? v.y : (c == 1 ? v.z : v.w);
-        }
-      }
-      if (want_phi && potential != nullptr) {
-        for (int e = threadIdx.x; e < kn * nu; e += blockDim.x) {
+      __syncthreads();
+      if (layout == 1) {
+#pragma unroll 4
+        for (int e = threadIdx.x; e < kn * nu; e += 256) {
           const int k = e / nu;
           const int t = e - k * nu;
-          potential[static_cast<long long>(kc + k) * nt + u0 + t] = tile[t][k].x;
+          reinterpret_cast<float4 *>(field)[static_cast<long long>(kc + k) * nt + u0 + t] = tile[t][k];
+        }
+      } else {
+        if (want_h) {
+#pragma unroll 4
+          for (int e = threadIdx.x; e < kn * nu * 3; e += 256) {
+            const int k = e / (nu * 3);
+            const int r = e - k * (nu * 3);
+            const int t = r / 3;
+            const int c = r - 3 * t;
+            field[(static_cast<long long>(kc + k) * nt + u0) * 3 + r] =
+                reinterpret_cast<const float *>(&tile[t][k])[1 + c];
+          }
+        }
+        if (want_phi && potential != nullptr) {
+#pragma unroll 4
+          for (int e = threadIdx.x; e < kn * nu; e += 256) {
+            const int k = e / nu;
+            const int t = e - k * nu;
+            potential[static_cast<long long>(kc + k) * nt + u0 + t] = tile[t][k].x;
+          }
         }
       }
-    }
-    __syncthreads();
-  }
+      __syncthreads();
+    });
 }
 
 // Position gradient of L = sum_k w_k . H_k (reverse mode; no counterpart in
